@@ -408,9 +408,9 @@ int llb_event_elapsed_ms(llb_handle h, int32_t slot_begin, int32_t slot_end, flo
 /* Step-kernel selection, for the autotuner.  Plain steps run the TMA-pipelined
    kernel in configuration `config` (0..2: tile shape, stage count, warps; 6:
    the form's default shape with the tile's bounce bytes loaded too), the
-   two-steps-per-pass kernel (3..5: the intermediate step stays in shared
-   memory, so a pair of steps reads and writes the populations once; a lone
-   step runs on the one-thread kernel), the one-thread-per-node kernel for
+   two-steps-per-pass kernel (3..5: the intermediate step stays in registers,
+   so a pair of steps reads and writes the populations once; a lone step runs
+   on the one-thread kernel), the one-thread-per-node kernel for
    config -1, for config -2 one thread per node of every 32-byte population
    sector that holds an active node (a list built on first use), for config -3
    one thread per slot of compacted planes that store only the fluid and open

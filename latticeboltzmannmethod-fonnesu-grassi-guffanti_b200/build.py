@@ -28,6 +28,7 @@ COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-O2", "-I", CSR
 SOURCES = {
     "llb_f64.cu": ["--fmad=false"],
     "llb_lowp.cu": ["--fmad=false"],
+    "llb_stream.cu": ["--fmad=false"],
     "llb_capi.cu": [],
     "llb_noalloc.cu": [],
     "llb_batch.cu": [],

@@ -321,11 +321,36 @@ int build_maps(llb_handle h) {
     return LLB_OK;
 }
 
-// Steps one plain-step launch advances: 2 for the two-step configurations.
-int steps_per_launch(llb_handle h) {
-    TmaPlan p;
-    return h->tma_cfg >= 0 && tma_plan(h->storage, h->tma_cfg, &p) && p.pair ? 2 : 1;
+// Tensor maps of the two population buffers, (ld, C, 9) elements in boxes of
+// stream_box_rows x 1 x 9: a column of a strip, all directions.
+int build_stream_maps(llb_handle h, int cfg) {
+    if (h->stream_maps == cfg) return LLB_OK;
+    auto enc = tensor_map_encoder();
+    if (!enc) return fail(h, LLB_E_CUDA, "cuTensorMapEncodeTiled unavailable");
+    const CUtensorMapDataType dt = h->storage == LLB_STORE_F64   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
+                                   : h->storage == LLB_STORE_F32S ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                                                  : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(h->ld), static_cast<cuuint64_t>(h->C), 9};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(h->ld) * h->elem, static_cast<cuuint64_t>(h->plane) * h->elem};
+    const cuuint32_t box[3] = {static_cast<cuuint32_t>(stream_box_rows(h->storage, cfg)), 1, 9};
+    const cuuint32_t es[3] = {1, 1, 1};
+    for (int b = 0; b < 2; ++b) {
+        CUresult r = enc(&h->smap[b], dt, 3, h->f[b], dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(h, LLB_E_CUDA, "cuTensorMapEncodeTiled (strips) failed");
+    }
+    h->stream_maps = cfg;
+    return LLB_OK;
 }
+
+// The plain-step kernel of a run of `plain` steps: the handle's configuration,
+// or the streaming kernel on lattices whose default groups longer runs.
+int run_config(llb_handle h, int32_t plain) {
+    return h->group_min > 0 && plain >= h->group_min ? FIRST_STREAM_CONFIG : h->tma_cfg;
+}
+
+// Steps one plain-step launch of a configuration advances.
+int steps_per_launch(int cfg) { return is_stream(cfg) ? STREAM_STEPS : 1; }
 
 // ---------------------------------------------------------------------------
 // column-compacted storage (pipeline PIPE_COMPACT)
@@ -527,37 +552,42 @@ bool cluster_ok(llb_handle h) {
     return h->cl_state > 0;
 }
 
-// One step kernel (two steps for a two-step configuration unless `single`).
-// Inside a graph capture the step index is relative (graph_offset >= 0, base
-// read from d_step); otherwise it is absolute.
-int launch_one(llb_handle h, bool macro, long long graph_offset = -1, bool single = false) {
+// One launch of the step kernel of configuration cfg (two steps for a streaming
+// one), or one output step.  Inside a graph capture the step index is relative
+// (graph_offset >= 0, base read from d_step); otherwise it is absolute.
+int launch_one(llb_handle h, int cfg, bool macro, long long graph_offset = -1) {
     LaunchCtx x = make_ctx(h);
     if (graph_offset >= 0) {
         x.ss.tbase = h->d_step;
         x.ss.t_off = graph_offset;
     }
-    if (!macro && h->tma_cfg == PIPE_COMPACT) {
+    if (!macro && cfg == PIPE_COMPACT) {
         cudaError_t e = launch_step_compact(h->storage, x, compact_geo(h), h->cf[h->cur], h->cf[h->cur ^ 1]);
         if (e != cudaSuccess) return cuda_fail(h, e, "compacted step kernel launch");
         h->cur ^= 1;
         ++h->step;
         return LLB_OK;
     }
-    if (!macro && h->tma_cfg >= 0) {
+    if (!macro && is_stream(cfg)) {
+        int rc = build_stream_maps(h, cfg);
+        if (rc) return rc;
+        cudaError_t e = launch_step_stream(h->storage, cfg, x, &h->smap[h->cur], h->f[h->cur ^ 1], h->sm_count);
+        if (e != cudaSuccess) return cuda_fail(h, e, "streaming step kernel launch");
+        h->cur ^= 1;
+        h->step += STREAM_STEPS;
+        return LLB_OK;
+    }
+    if (!macro && cfg >= 0) {
         int rc = build_maps(h);
         if (rc) return rc;
-        if (!(h->plan.pair && single)) {
-            const long long ntiles =
-                ((h->R + h->plan.TI - 1) / h->plan.TI) * ((h->C + h->plan.TJ - 1) / h->plan.TJ);
-            const int grid = static_cast<int>(std::min<long long>(ntiles, static_cast<long long>(h->sm_count) * h->plan.ctas_per_sm));
-            cudaError_t e = launch_step_tma(h->storage, h->plan, x, &h->pmap[h->cur], &h->mmap, &h->bmap,
-                                            h->f[h->cur], h->f[h->cur ^ 1], grid);
-            if (e != cudaSuccess) return cuda_fail(h, e, "pipelined step kernel launch");
-            h->cur ^= 1;
-            h->step += h->plan.pair ? 2 : 1;
-            return LLB_OK;
-        }
-        // a lone step of a two-step configuration: the one-thread-per-node kernel
+        const long long ntiles = ((h->R + h->plan.TI - 1) / h->plan.TI) * ((h->C + h->plan.TJ - 1) / h->plan.TJ);
+        const int grid = static_cast<int>(std::min<long long>(ntiles, h->sm_count));
+        cudaError_t e = launch_step_tma(h->storage, h->plan, x, &h->pmap[h->cur], &h->mmap, &h->bmap, h->f[h->cur],
+                                        h->f[h->cur ^ 1], grid);
+        if (e != cudaSuccess) return cuda_fail(h, e, "pipelined step kernel launch");
+        h->cur ^= 1;
+        ++h->step;
+        return LLB_OK;
     }
     cudaError_t e = launch_step(h->storage, x, h->f[h->cur], h->f[h->cur ^ 1], false, macro);
     if (e != cudaSuccess) return cuda_fail(h, e, "step kernel launch");
@@ -573,8 +603,8 @@ int graph_for(llb_handle h, cudaGraphExec_t* out) {
     cudaGraph_t g = nullptr;
     LLB_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int rc = LLB_OK;
-    const int per = steps_per_launch(h);
-    for (int s = 0; s < GRAPH_STEPS && rc == LLB_OK; s += per) rc = launch_one(h, false, s);
+    const int cfg = run_config(h, GRAPH_STEPS), per = steps_per_launch(cfg);
+    for (int s = 0; s < GRAPH_STEPS && rc == LLB_OK; s += per) rc = launch_one(h, cfg, false, s);
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
     h->cur = cur0;
     h->step = step0;
@@ -837,6 +867,7 @@ int llb_create(const llb_desc* d, llb_handle* out) {
         h->tma_cfg = default_dense_pipeline(*h);
         h->err.clear();
     }
+    h->group_min = default_group_min(*h);
     *out = h;
     return LLB_OK;
 }
@@ -892,10 +923,11 @@ int llb_step(llb_handle h, int32_t nsteps, uint32_t flags) {
     if (rc) return rc;
     const bool macro = (flags & LLB_STEP_MACRO) != 0;
     int32_t plain = macro ? nsteps - 1 : nsteps;
-    const bool compact = h->tma_cfg == PIPE_COMPACT;
+    const int cfg = run_config(h, plain);
+    const bool compact = cfg == PIPE_COMPACT;
     if (plain > 0 && (rc = compact ? state_to_compact(h) : state_to_dense(h))) return rc;
     if (plain > 0) h->where = compact ? RES_COMPACT : RES_DENSE;  // where the steps below leave it
-    if (plain >= GRAPH_STEPS && h->tma_cfg != PIPE_CLUSTER) {
+    if (plain >= GRAPH_STEPS && cfg != PIPE_CLUSTER) {
         cudaGraphExec_t g = nullptr;
         if ((rc = graph_for(h, &g))) return rc;
         while (plain >= GRAPH_STEPS) {
@@ -906,7 +938,7 @@ int llb_step(llb_handle h, int32_t nsteps, uint32_t flags) {
             plain -= GRAPH_STEPS;
         }
     }
-    if (h->tma_cfg == PIPE_CLUSTER) {
+    if (cfg == PIPE_CLUSTER) {
         // chunks of steps, each one launch of the cluster
         while (plain > 0) {
             const int n = std::min<int32_t>(plain, CLUSTER_CHUNK);
@@ -918,14 +950,18 @@ int llb_step(llb_handle h, int32_t nsteps, uint32_t flags) {
             plain -= n;
         }
     }
-    const int per = steps_per_launch(h);
+    const int per = steps_per_launch(cfg);
     for (; plain >= per; plain -= per)
-        if ((rc = launch_one(h, false))) return rc;
-    if (plain > 0 && (rc = launch_one(h, false, -1, true))) return rc;
+        if ((rc = launch_one(h, cfg, false))) return rc;
+    // a lone step left over by a two-step configuration: the handle's own dense
+    // kernel, else one thread per node
+    const int lone = is_stream(h->tma_cfg) || h->tma_cfg == PIPE_COMPACT ? PIPE_GRID : h->tma_cfg;
+    for (; plain > 0; --plain)
+        if ((rc = launch_one(h, lone, false))) return rc;
     if (macro) {
         // output steps write rho and u from the dense kernel
         if ((rc = state_to_dense(h))) return rc;
-        if ((rc = launch_one(h, true))) return rc;
+        if ((rc = launch_one(h, h->tma_cfg, true))) return rc;
         h->where = RES_DENSE;
         h->macro_valid = true;
     }
@@ -1198,7 +1234,7 @@ int llb_set_pipeline(llb_handle h, int32_t config) {
         if (!cluster_ok(h))
             return fail(h, LLB_E_UNSUPPORTED, "the lattice's column slabs do not fit the shared memory of one cluster");
     }
-    if (config != h->tma_cfg) {
+    if (config != h->tma_cfg || h->group_min > 0) {
         int rc = select_device(h);
         if (rc) return rc;
         if (config == PIPE_LIST && (rc = build_sector_list(h))) return rc;
@@ -1208,7 +1244,9 @@ int llb_set_pipeline(llb_handle h, int32_t config) {
         for (auto& g : h->graph)
             if (g) { cudaGraphExecDestroy(g); g = nullptr; }
         h->tma_cfg = config;
+        h->group_min = 0;
         h->maps_ready = false;
+
     }
     return LLB_OK;
 }

@@ -70,6 +70,12 @@ struct llb_lattice {
     TmaPlan plan;
     bool maps_ready = false;
     CUtensorMap pmap[2];  // populations f[0], f[1]
+    int stream_maps = -1;  // the streaming configuration smap was built for
+    CUtensorMap smap[2];   // populations in the boxes of the streaming kernel
+    // runs of at least this many plain steps use the streaming kernel (two steps
+    // per pass) whatever tma_cfg says; 0: never.  Set by default on large
+    // lattices, cleared by llb_set_pipeline.
+    int group_min = 0;
     CUtensorMap mmap;     // node mask
     CUtensorMap bmap;     // bounce bytes (configurations that load them)
     int sm_count = 148;
@@ -119,7 +125,8 @@ constexpr int RES_DENSE = 0, RES_COMPACT = 1, RES_BOTH = 2;
 //    3, from 2^28 bytes), the TMA pipeline for FP16 (from 2^27 bytes); else
 //    one thread per node, which runs close to the copy bandwidth on open flow
 //    (there every node is active and the compacted planes only add their
-//    6 bytes of addressing per node);
+//    6 bytes of addressing per node).  This is the kernel of a lone step;
+//    longer runs may take the streaming kernel (default_group_min);
 //  * lattices resident in one 16-block cluster (their slabs fit its shared
 //    memory) up to 12 000 nodes (FP64, FP32) or 26 000 (FP16): the cluster
 //    runs a chunk of steps per launch (chosen at creation, where the device
@@ -145,11 +152,32 @@ inline int default_dense_pipeline(const llb_lattice& h) {
         return h.storage == LLB_STORE_F64 ? (n >= (int64_t{1} << 21) ? 1 : 0) : 6;
     const double state = 2.0 * 9.0 * static_cast<double>(h.elem) * static_cast<double>(n);
     if (h.storage == LLB_STORE_F16S) return state >= static_cast<double>(int64_t{1} << 27) ? 0 : PIPE_GRID;
-    return state >= static_cast<double>(int64_t{1} << 28) ? llb::FIRST_PAIR_CONFIG : PIPE_GRID;
+    return state >= static_cast<double>(int64_t{1} << 28) ? llb::FIRST_STREAM_CONFIG : PIPE_GRID;
 }
 inline int default_pipeline(const llb_lattice& h) {
     if (obstacle_rich(h) && h.R * h.C >= COMPACT_MIN_NODES) return PIPE_COMPACT;
     return default_dense_pipeline(h);
+}
+// Runs of at least this many plain steps take the streaming kernel, two steps
+// per pass (llb_stream.cuh), on lattices whose state no longer sits in L2; 0
+// where they never do.  Measured on B200, us a step, default kernel / streaming:
+//   cavity FP64  724^2 9.3 / 10.3, 850^2 15.5 / 13.0, 1000^2 23.3 / 18.2
+//          FP32  850^2 8.7 / 9.1, 512 x 2048 12.2 / 11.5, 1200^2 18.6 / 15.0
+//          FP16  850^2 9.8 / 10.0, 1000^2 12.7 / 10.8, 2048^2 49.4 / 33.1
+//   porous (against the compacted planes, which read 30 % fewer nodes)
+//          FP64  1448^2 37.3 / 38.1, 2048^2 70.4 / 67.7, 4096^2 268 / 250
+//          FP32  1024^2 10.0 / 12.7, 1448^2 23.4 / 21.0, 4096^2 162 / 128
+//          FP16  1500 x 2000 26.7 / 27.6, 2048^2 39.9 / 36.6, 4096^2 142 / 119
+// On the compacted pipeline only longer runs leave its planes: shorter ones
+// would pay for the copies between the layouts.
+inline int default_group_min(const llb_lattice& h) {
+    if (h.d_ps || h.n_active == 0) return 0;
+    const int64_t n = h.R * h.C;
+    const int form = h.storage == LLB_STORE_F64 ? 0 : h.storage == LLB_STORE_F32S ? 1 : 2;
+    static constexpr int64_t kDense[3] = {5LL << 17, 8LL << 17, 7LL << 17};
+    static constexpr int64_t kPorous[3] = {3LL << 20, 2LL << 20, 4LL << 20};
+    if (h.tma_cfg == PIPE_COMPACT) return n >= kPorous[form] ? 32 : 0;
+    return n >= kDense[form] ? llb::STREAM_STEPS : 0;
 }
 
 namespace llb {

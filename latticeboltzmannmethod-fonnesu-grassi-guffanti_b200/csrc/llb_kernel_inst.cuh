@@ -4,29 +4,12 @@
 #include "llb_kernels.cuh"
 #include "llb_launch.h"
 #include "llb_tma.cuh"
-#include "llb_pair.cuh"
 #include "llb_batch.cuh"
 #include "llb_compact.cuh"
 #include "llb_cluster.cuh"
+#include "llb_pdl.cuh"
 
 namespace llb {
-
-// Launch of kernel k with programmatic stream serialization (the kernel waits
-// for the previous one itself: pdl_wait_then_release).
-template <class... KArgs, class... Args>
-cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, cudaStream_t stream, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, args...);
-}
 
 template <class M>
 cudaError_t do_step(const LaunchCtx& x, const void* fin, void* fout, bool init, bool macro) {
@@ -234,9 +217,7 @@ cudaError_t do_gather(const LaunchCtx& x, const void* fin, const int64_t* pts, c
 template <class M, class CFG>
 void fill_plan(int cfg, TmaPlan* p) {
     p->cfg = cfg;
-    p->pair = CFG::PAIR;
-    p->ctas_per_sm = CFG::CPS;
-    if constexpr (!CFG::PAIR) p->bbx = CFG::BBX;
+    p->bbx = CFG::BBX;
     p->TI = CFG::TI;
     p->TJ = CFG::TJ;
     p->S = CFG::S;
@@ -257,23 +238,6 @@ cudaError_t do_step_tma(const LaunchCtx& x, const CUtensorMap* pmap, const CUten
     auto k1 = k_step_tma<M, 1, CFG>;
     auto kern = x.c.model == 0 ? k0 : k1;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CFG::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    kern<<<grid, CFG::THREADS, CFG::SMEM_BYTES, x.stream>>>(*pmap, *mmap, *bmap, x.g, x.ot, x.c,
-                                                             static_cast<const T*>(fin), static_cast<T*>(fout), x.ss);
-    return cudaGetLastError();
-}
-
-template <class M, class CFG>
-cudaError_t do_step_pair(const LaunchCtx& x, const CUtensorMap* pmap, const CUtensorMap* mmap,
-                         const CUtensorMap* bmap, const void* fin, void* fout, int grid) {
-    using T = typename M::T;
-    auto k0 = k_step_pair<M, 0, CFG>;
-    auto k1 = k_step_pair<M, 1, CFG>;
-    auto kern = x.c.model == 0 ? k0 : k1;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CFG::SMEM_BYTES);
-    // CFG::CPS CTAs of this kernel share an SM's shared memory
-    if (e == cudaSuccess && CFG::CPS > 1)
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     kern<<<grid, CFG::THREADS, CFG::SMEM_BYTES, x.stream>>>(*pmap, *mmap, *bmap, x.g, x.ot, x.c,
                                                              static_cast<const T*>(fin), static_cast<T*>(fout), x.ss);

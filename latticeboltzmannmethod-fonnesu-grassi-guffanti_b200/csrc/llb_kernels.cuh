@@ -69,25 +69,31 @@ __device__ __forceinline__ void pull(const Geometry& g, const typename M::T* __r
     }
 }
 
+// Row of the boundary-value ring that holds step t (one row: values constant in
+// time, and no 64-bit division on the node's path).
+__device__ __forceinline__ long long open_row(const OpenTable& ot, long long t) {
+    return ot.cap == 1 ? 0LL : t % ot.cap;
+}
+
 // Closure + choice of (rho, u) for an open node at step t (t >= 1), or for the
 // initial step (t == 0: no closure, pressure nodes start at rest).
 template <class M>
 __device__ __forceinline__ void open_node(const OpenTable& ot, int q, uint8_t m, long long t, typename M::R* f,
                                           double& rho, double& ux, double& uy) {
     const int side = mask_side(m), bc = mask_bc(m);
-    const double2 cur = ot.vals[static_cast<long long>(t % ot.cap) * ot.n_open + q];
+    const double2 cur = ot.vals[open_row(ot, t) * ot.n_open + q];
     if (bc == BC_ZH_PRES) {
         rho = cur.x;
         if (t == 0) {
             ux = 0.0;
             uy = 0.0;
         } else {
-            const double2 prev = ot.vals[static_cast<long long>((t - 1) % ot.cap) * ot.n_open + q];
+            const double2 prev = ot.vals[open_row(ot, t - 1) * ot.n_open + q];
             M::closure_pressure(f, side, prev.x, prev.y, ux, uy);
         }
     } else {
         if (bc == BC_ZH_VEL && t > 0) {
-            const double2 prev = ot.vals[static_cast<long long>((t - 1) % ot.cap) * ot.n_open + q];
+            const double2 prev = ot.vals[open_row(ot, t - 1) * ot.n_open + q];
             M::closure_velocity(f, side, prev.x, prev.y);
         }
         rho = 1.0;  // open nodes collide with global_rho == 1 (never written for them)
@@ -343,7 +349,7 @@ __global__ void __launch_bounds__(BX* BY) k_finalize(Geometry g, OpenTable ot, c
     pull<M>(g, fin, i, j, node, m, false, f);
     if (cls == CLS_OPEN && t > 0) {
         const int q = g.open_idx[node];
-        const double2 prev = ot.vals[static_cast<long long>((t - 1) % ot.cap) * ot.n_open + q];
+        const double2 prev = ot.vals[open_row(ot, t - 1) * ot.n_open + q];
         if (mask_bc(m) == BC_ZH_VEL) M::closure_velocity(f, mask_side(m), prev.x, prev.y);
         else if (mask_bc(m) == BC_ZH_PRES) {
             double ux, uy;

@@ -62,6 +62,17 @@ cudaError_t launch_step_cluster_f64(const LaunchCtx&, const ClusterPlan&, void*,
 cudaError_t launch_step_cluster_lowp(int storage, const LaunchCtx&, const ClusterPlan&, void*, void*, int, long long,
                                      int);
 
+// STREAM_STEPS plain steps per launch, streamed through registers
+// (llb_stream.cuh; configurations FIRST_STREAM_CONFIG .. +2).  pmap: the
+// population planes in boxes of stream_box_rows rows x 1 column x 9 planes.
+// False / an error for lattices beyond its 32-bit column offsets.
+constexpr int STREAM_STEPS = 2;
+constexpr int FIRST_STREAM_CONFIG = 3;
+constexpr bool is_stream(int cfg) { return cfg >= FIRST_STREAM_CONFIG && cfg < FIRST_STREAM_CONFIG + 3; }
+int stream_box_rows(int storage, int cfg);
+cudaError_t launch_step_stream(int storage, int cfg, const LaunchCtx& ctx, const CUtensorMap* pmap, void* fout,
+                               int sm_count);
+
 struct BatchLattice;
 // Batched step over a work list (llb_batch.cuh).  `cooperative` launches the
 // grid cooperatively (required when steps > 1).
@@ -116,8 +127,6 @@ cudaError_t launch_gather_forces_lowp(int storage, const LaunchCtx&, const void*
 // S shared-memory stages, W consumer warps + 1 producer warp).
 struct TmaPlan {
     int cfg = -1;
-    bool pair = false;     // two steps per launch (k_step_pair)
-    int ctas_per_sm = 1;   // persistent grid = ctas_per_sm x SM count
     bool bbx = false;      // the producer also loads a TI x TJ box of bounce bytes
     int TI = 0, TJ = 0, S = 0, W = 0;
     int BI = 0;            // rows of a population box
@@ -127,10 +136,9 @@ struct TmaPlan {
     int threads = 0;
 };
 // Configurations 0..2 and 6: one step per launch (k_step_tma; 6 also loads the
-// tile's bounce bytes); 3..5: two steps per launch (k_step_pair).
+// tile's bounce bytes); 3..5: two steps per launch (k_step_stream).
 constexpr int TMA_CONFIGS = 7;
-constexpr int FIRST_PAIR_CONFIG = 3;
-// Fills `out` for configuration `cfg` (0..TMA_CONFIGS-1) of a storage form.
+// Fills `out` for configuration `cfg` (0..2 or 6) of a storage form; false for any other.
 bool tma_plan(int storage, int cfg, TmaPlan* out);
 cudaError_t launch_step_tma(int storage, const TmaPlan& p, const LaunchCtx& ctx, const CUtensorMap* pmap,
                             const CUtensorMap* mmap, const CUtensorMap* bmap, const void* fin, void* fout, int grid);

@@ -27,11 +27,16 @@ struct ModelF64 {
     static __device__ __forceinline__ double to_f64(R v, int) { return v; }
 
     // DefaultEquilibrium<2>::update_macro (DefaultEquilibrium.hpp:135-153)
-    static __device__ __forceinline__ void moments(const R* p, R& rho, R& ux, R& uy) {
-        rho = p[0] + p[1] + p[2] + p[3] + p[4] + p[5] + p[6] + p[7] + p[8];
-        const double rhoinv = 1.0 / rho;
+    static __device__ __forceinline__ R density(const R* p) {
+        return p[0] + p[1] + p[2] + p[3] + p[4] + p[5] + p[6] + p[7] + p[8];
+    }
+    static __device__ __forceinline__ void velocity(const R* p, R rhoinv, R& ux, R& uy) {
         ux = rhoinv * (p[1] + p[5] + p[8] - (p[3] + p[6] + p[7]));
         uy = rhoinv * (p[2] + p[5] + p[6] - (p[4] + p[7] + p[8]));
+    }
+    static __device__ __forceinline__ void moments(const R* p, R& rho, R& ux, R& uy) {
+        rho = density(p);
+        velocity(p, 1.0 / rho, ux, uy);
     }
 
     // ZouHePolicy<2>::update_boundaries (ZouHePolicy.hpp:70-118); ux, uy are the
@@ -179,6 +184,70 @@ struct ModelF64 {
 // The closures are unchanged in g because opposite directions share weights;
 // only the density sums carry the constant (sum of the weights involved = 1).
 // ============================================================================
+
+// FP32 arithmetic on one node (One) or on two nodes at a time (Two: the packed
+// FP32 instructions of sm_100, one issue slot for two nodes).  Every operation
+// rounds to nearest on each node alone, so both give the same bits.
+struct One {
+    using V = float;
+    static __device__ __forceinline__ V all(float a) { return a; }
+    static __device__ __forceinline__ V add(V a, V b) { return __fadd_rn(a, b); }
+    static __device__ __forceinline__ V sub(V a, V b) { return __fsub_rn(a, b); }
+    static __device__ __forceinline__ V mul(V a, V b) { return __fmul_rn(a, b); }
+    static __device__ __forceinline__ V fma(V a, V b, V c) { return __fmaf_rn(a, b, c); }
+};
+struct Two {
+    using V = unsigned long long;
+    static __device__ __forceinline__ V pack(float a, float b) {
+        V r;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+        return r;
+    }
+    static __device__ __forceinline__ float2 unpack(V v) {
+        float2 r;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+        return r;
+    }
+    static __device__ __forceinline__ V all(float a) { return pack(a, a); }
+    static __device__ __forceinline__ V add(V a, V b) {
+        V r;
+        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+        return r;
+    }
+    static __device__ __forceinline__ V sub(V a, V b) { return fma(b, all(-1.0f), a); }
+    static __device__ __forceinline__ V mul(V a, V b) {
+        V r;
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+        return r;
+    }
+    static __device__ __forceinline__ V fma(V a, V b, V c) {
+        V r;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+        return r;
+    }
+    // 1 / a, rounded as the division rounds it, for 2^-120 < a < 2^120: one
+    // Newton step on the approximate reciprocal gives the rounded quotient
+    // (Markstein, IBM J. Res. Dev. 34, 1990); compared with 1.0f / x for every
+    // 32-bit pattern on B200, equal for all exponents from -126 to 125.
+    static __device__ __forceinline__ V inverse_mid(V a) {
+        const float2 x = unpack(a);
+        float yx, yy;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yx) : "f"(x.x));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yy) : "f"(x.y));
+        const V y = pack(yx, yy);
+        const V na = mul(a, all(-1.0f));
+        return fma(y, fma(na, y, all(1.0f)), y);
+    }
+    static __device__ __forceinline__ V inverse(V a) {
+        const float2 x = unpack(a);
+        return pack(1.0f / x.x, 1.0f / x.y);
+    }
+    static __device__ __forceinline__ bool mid(V a) {
+        const float2 x = unpack(a);
+        return fminf(x.x, x.y) > 0x1p-120f && fmaxf(x.x, x.y) < 0x1p120f;
+    }
+};
+
 template <typename TS>
 struct ModelShift {
     using T = TS;
@@ -195,12 +264,23 @@ struct ModelShift {
     }
     static __device__ __forceinline__ double to_f64(R v, int k) { return static_cast<double>(v) + w_init(k); }
 
-    // returns rho - 1 in rho (kept small for precision)
+    // rho - 1 (kept small for precision)
+    template <class A>
+    static __device__ __forceinline__ typename A::V density_of(const typename A::V* g) {
+        return A::add(A::add(A::add(A::add(g[0], g[1]), A::add(g[2], g[3])),
+                             A::add(A::add(g[4], g[5]), A::add(g[6], g[7]))),
+                      g[8]);
+    }
+    // inv: 1 / rho
+    template <class A>
+    static __device__ __forceinline__ void velocity_of(const typename A::V* g, typename A::V inv, typename A::V& ux,
+                                                       typename A::V& uy) {
+        ux = A::mul(inv, A::sub(A::add(A::add(g[1], g[5]), g[8]), A::add(A::add(g[3], g[6]), g[7])));
+        uy = A::mul(inv, A::sub(A::add(A::add(g[2], g[5]), g[6]), A::add(A::add(g[4], g[7]), g[8])));
+    }
     static __device__ __forceinline__ void moments(const R* g, R& drho, R& ux, R& uy) {
-        drho = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + (g[6] + g[7])) + g[8];
-        const R inv = 1.0f / (1.0f + drho);
-        ux = inv * ((g[1] + g[5] + g[8]) - (g[3] + g[6] + g[7]));
-        uy = inv * ((g[2] + g[5] + g[6]) - (g[4] + g[7] + g[8]));
+        drho = density_of<One>(g);
+        velocity_of<One>(g, 1.0f / (1.0f + drho), ux, uy);
     }
 
     static __device__ __forceinline__ void close(R* g, int side, R ru, R rv) {
@@ -273,47 +353,52 @@ struct ModelShift {
     // BGK or TRT on the shifted values (the shifts cancel in both operators).
     // Opposite directions k, opp(k) share w_k and cu^2 and differ in the sign
     // of cu, so each pair is computed once: g_eq = w (even +- odd).
-    template <int COLL>
-    static __device__ __forceinline__ void collide(R* g, R drho, R ux, R uy, const Collision& c) {
-        // multiply-adds written out (__fmaf_rn): the translation unit is built
-        // without automatic contraction, so every kernel rounds alike
-        const R rho = 1.0f + drho;
-        const R u2 = 1.5f * __fmaf_rn(ux, ux, uy * uy);
-        const R e0 = w_f32(0) * __fmaf_rn(-rho, u2, drho);
+    template <int COLL, class A>
+    static __device__ __forceinline__ void collide_of(typename A::V* g, typename A::V drho, typename A::V ux,
+                                                      typename A::V uy, const Collision& c) {
+        using V = typename A::V;
+        // multiply-adds written out: the translation unit is built without
+        // automatic contraction, so every kernel rounds alike
+        const V rho = A::add(A::all(1.0f), drho);
+        const V nu2 = A::mul(A::all(-1.5f), A::fma(ux, ux, A::mul(uy, uy)));
+        const V e0 = A::mul(A::all(w_f32(0)), A::fma(rho, nu2, drho));
         // pairs (1,3), (2,4), (5,7), (6,8): cu of the first direction of each pair
-        // (DJ, DI are 0 or +-1, so cu is a sum or difference of ux and uy)
         constexpr int first[4] = {1, 2, 5, 6};
-        R ev[4], od[4];
+        const V cu[4] = {ux, uy, A::add(ux, uy), A::sub(uy, ux)};
+        V ev[4], od[4];
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
-            const int k = first[p];
-            const R cu = static_cast<R>(DJ(k)) * ux - static_cast<R>(DI(k)) * uy;
-            ev[p] = w_f32(k) * __fmaf_rn(rho, __fmaf_rn(4.5f * cu, cu, -u2), drho);
-            od[p] = w_f32(k) * (rho * (3.0f * cu));
+            const V w = A::all(w_f32(first[p]));
+            ev[p] = A::mul(w, A::fma(rho, A::fma(A::mul(A::all(4.5f), cu[p]), cu[p], nu2), drho));
+            od[p] = A::mul(w, A::mul(rho, A::mul(A::all(3.0f), cu[p])));
         }
         if (COLL == 0) {
-            const R t = c.tf, omt = c.omtf;
-            g[0] = __fmaf_rn(omt, g[0], t * e0);
+            const V t = A::all(c.tf), omt = A::all(c.omtf);
+            g[0] = A::fma(omt, g[0], A::mul(t, e0));
 #pragma unroll
             for (int p = 0; p < 4; ++p) {
                 const int k = first[p], b = opp(k);
-                g[k] = __fmaf_rn(omt, g[k], t * (ev[p] + od[p]));
-                g[b] = __fmaf_rn(omt, g[b], t * (ev[p] - od[p]));
+                g[k] = A::fma(omt, g[k], A::mul(t, A::add(ev[p], od[p])));
+                g[b] = A::fma(omt, g[b], A::mul(t, A::sub(ev[p], od[p])));
             }
         } else {
-            const R ie = c.ief, he = c.hef, ho = c.hof;
-            g[0] = __fmaf_rn(-ie, g[0] - e0, g[0]);
+            const V nie = A::all(-c.ief), nhe = A::all(-c.hef), ho = A::all(c.hof), nho = A::all(-c.hof);
+            g[0] = A::fma(nie, A::sub(g[0], e0), g[0]);
 #pragma unroll
             for (int p = 0; p < 4; ++p) {
                 const int k = first[p], b = opp(k);
                 // symmetric and antisymmetric non-equilibrium parts of the pair
-                const R sym = __fmaf_rn(-2.0f, ev[p], g[k] + g[b]);
-                const R asym = __fmaf_rn(-2.0f, od[p], g[k] - g[b]);
-                const R qk = g[k], qb = g[b];
-                g[k] = __fmaf_rn(-ho, asym, __fmaf_rn(-he, sym, qk));
-                g[b] = __fmaf_rn(ho, asym, __fmaf_rn(-he, sym, qb));
+                const V sym = A::fma(A::all(-2.0f), ev[p], A::add(g[k], g[b]));
+                const V asym = A::fma(A::all(-2.0f), od[p], A::sub(g[k], g[b]));
+                const V qk = g[k], qb = g[b];
+                g[k] = A::fma(nho, asym, A::fma(nhe, sym, qk));
+                g[b] = A::fma(ho, asym, A::fma(nhe, sym, qb));
             }
         }
+    }
+    template <int COLL>
+    static __device__ __forceinline__ void collide(R* g, R drho, R ux, R uy, const Collision& c) {
+        collide_of<COLL, One>(g, drho, ux, uy, c);
     }
 
     static __device__ __forceinline__ double rho_f64(R drho) { return 1.0 + static_cast<double>(drho); }

@@ -387,7 +387,9 @@ class CudaLattice:
         planes (active nodes only); -4: the lattice resident in one
         thread-block cluster's shared memory, a chunk of steps per launch;
         0..2 and 6: TMA pipeline configurations (6 also loads the tile's
-        bounce bytes); 3..5: two steps per pass through shared memory."""
+        bounce bytes); 3..5: two steps per pass, streamed through registers.
+        Without this call a large lattice runs its longer runs two steps per
+        pass whatever `pipeline` says of its lone steps."""
         _check(lib().llb_set_pipeline(self._h, config), self._h)
 
     @property
