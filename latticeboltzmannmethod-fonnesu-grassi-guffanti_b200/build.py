@@ -29,6 +29,7 @@ SOURCES = {
     "llb_f64.cu": ["--fmad=false"],
     "llb_lowp.cu": ["--fmad=false"],
     "llb_stream.cu": ["--fmad=false"],
+    "llb_tile.cu": ["--fmad=false"],
     "llb_capi.cu": [],
     "llb_noalloc.cu": [],
     "llb_batch.cu": [],

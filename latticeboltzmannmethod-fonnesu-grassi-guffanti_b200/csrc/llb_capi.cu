@@ -596,6 +596,26 @@ int launch_one(llb_handle h, int cfg, bool macro, long long graph_offset = -1) {
     return LLB_OK;
 }
 
+// nsteps steps of a lattice that steps in tiles, several per launch, evenly
+// split; with macro the last one writes rho and u.
+int step_tiles(llb_handle h, int32_t nsteps, bool macro) {
+    int rc = state_to_dense(h);
+    if (rc) return rc;
+    for (int32_t left = nsteps; left > 0;) {
+        const int32_t launches = (left + h->tile.T - 1) / h->tile.T;
+        const int32_t k = (left + launches - 1) / launches;
+        const bool out = macro && k == left;
+        cudaError_t e = launch_step_tile(h->storage, make_ctx(h), h->tile, h->f[h->cur], h->f[h->cur ^ 1], k, out);
+        if (e != cudaSuccess) return cuda_fail(h, e, "tile step kernel launch");
+        h->cur ^= 1;
+        h->step += k;
+        left -= k;
+    }
+    h->where = RES_DENSE;
+    if (macro) h->macro_valid = true;
+    return LLB_OK;
+}
+
 int graph_for(llb_handle h, cudaGraphExec_t* out) {
     if (h->graph[h->cur]) { *out = h->graph[h->cur]; return LLB_OK; }
     const int cur0 = h->cur;
@@ -868,6 +888,8 @@ int llb_create(const llb_desc* d, llb_handle* out) {
         h->err.clear();
     }
     h->group_min = default_group_min(*h);
+    if (h->group_min == 0 && (h->tma_cfg == PIPE_GRID || h->tma_cfg == PIPE_CLUSTER))
+        (void)tile_plan(h->storage, static_cast<int>(h->R), static_cast<int>(h->C), !ps.empty(), h->sm_count, &h->tile);
     *out = h;
     return LLB_OK;
 }
@@ -922,6 +944,7 @@ int llb_step(llb_handle h, int32_t nsteps, uint32_t flags) {
     int rc = select_device(h);
     if (rc) return rc;
     const bool macro = (flags & LLB_STEP_MACRO) != 0;
+    if (h->tile.T > 0) return step_tiles(h, nsteps, macro);
     int32_t plain = macro ? nsteps - 1 : nsteps;
     const int cfg = run_config(h, plain);
     const bool compact = cfg == PIPE_COMPACT;
@@ -1234,7 +1257,7 @@ int llb_set_pipeline(llb_handle h, int32_t config) {
         if (!cluster_ok(h))
             return fail(h, LLB_E_UNSUPPORTED, "the lattice's column slabs do not fit the shared memory of one cluster");
     }
-    if (config != h->tma_cfg || h->group_min > 0) {
+    if (config != h->tma_cfg || h->group_min > 0 || h->tile.T > 0) {
         int rc = select_device(h);
         if (rc) return rc;
         if (config == PIPE_LIST && (rc = build_sector_list(h))) return rc;
@@ -1245,6 +1268,7 @@ int llb_set_pipeline(llb_handle h, int32_t config) {
             if (g) { cudaGraphExecDestroy(g); g = nullptr; }
         h->tma_cfg = config;
         h->group_min = 0;
+        h->tile = TilePlan{};
         h->maps_ready = false;
 
     }
@@ -1285,12 +1309,19 @@ int llb_tune_pipeline(llb_handle h, int32_t trial_steps, int32_t* best, float* m
         cudaEventDestroy(e0);
         return cuda_fail(h, ce, "cudaEventCreate");
     }
-    const int original = h->tma_cfg;
+    // the configuration the handle came with is timed as it steps by default
+    const int original = h->tma_cfg, group_min = h->group_min;
+    const TilePlan tile = h->tile;
+    auto by_default = [&] {
+        h->group_min = group_min;
+        h->tile = tile;
+    };
     int chosen = original;
     float chosen_ms = -1.0f;
     static constexpr int kCandidates[] = {PIPE_GRID, PIPE_LIST, PIPE_COMPACT, PIPE_CLUSTER, 0, 1, 2, 3, 4, 5, 6};
     for (int cfg : kCandidates) {
         if (llb_set_pipeline(h, cfg) != LLB_OK) continue;  // not available for this lattice
+        if (cfg == original) by_default();
         // warm-up (tensor maps, graphs), then the timed steps
         if ((rc = llb_step(h, trial_steps, 0))) break;
         cudaError_t te = cudaEventRecord(e0, h->stream);
@@ -1316,6 +1347,7 @@ int llb_tune_pipeline(llb_handle h, int32_t trial_steps, int32_t* best, float* m
     cudaEventDestroy(e1);
     if (rc) return rc;
     if ((rc = llb_set_pipeline(h, chosen))) return rc;
+    if (chosen == original) by_default();
     if (chosen != PIPE_LIST) release_sector_list(h);
     if (chosen != PIPE_COMPACT) release_compact(h);
     if (best) *best = chosen;

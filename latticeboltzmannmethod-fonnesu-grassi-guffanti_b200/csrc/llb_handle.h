@@ -105,6 +105,10 @@ struct llb_lattice {
     // fits, -1 it does not)
     llb::ClusterPlan cl_plan;
     int cl_state = 0;
+    // several steps per launch over register-resident tiles (llb_tile.cuh;
+    // T == 0: off): the plain and output steps of a lattice that fits L2 on its
+    // default kernel.  llb_set_pipeline turns it off.
+    llb::TilePlan tile;
 };
 
 // Residence of the state (llb_lattice::where).  Steps of the compacted
@@ -133,6 +137,7 @@ constexpr int RES_DENSE = 0, RES_COMPACT = 1, RES_BOTH = 2;
 //    is known).  96^2 steps in 2.2 us against 3.0 us on the one-thread grid;
 //    at config 1 (129^2) the 16 SMs of one cluster are bound by the FP64
 //    arithmetic of 16 641 nodes (3.6 us against 3.1 us), so the grid keeps it.
+//    Most of these lattices step in tiles anyway (tile_plan, llb_tile.cu).
 constexpr int PIPE_GRID = -1, PIPE_LIST = -2, PIPE_COMPACT = -3, PIPE_CLUSTER = -4;
 inline bool cluster_default_size(const llb_lattice& h) {
     return h.R * h.C <= (h.storage == LLB_STORE_F16S ? 26000 : 12000);

@@ -153,10 +153,11 @@ __device__ __forceinline__ double ps_equilibrium(int k, double rho, double ux, d
     }
 }
 
-// s: the node's populations before collision, f: after; bits: ps bits of the node.
-template <typename T>
-__device__ __forceinline__ void ps_push(const Geometry& g, T* __restrict__ fout, long long node, unsigned bits,
-                                        const double* s, const double* f, double rho, double ux, double uy, double t) {
+// s: the node's populations before collision, f: after; bits: ps bits of the
+// node; put(k, v) takes the value of direction k.
+template <class Put>
+__device__ __forceinline__ void ps_push_values(const Geometry& g, long long node, unsigned bits, const double* s,
+                                               const double* f, double rho, double ux, double uy, double t, Put put) {
     constexpr double one18 = (1.0 / 18.0);
     constexpr double one36 = (1.0 / 36.0);
 #pragma unroll
@@ -168,8 +169,14 @@ __device__ __forceinline__ void ps_push(const Geometry& g, T* __restrict__ fout,
         const double ek = ps_equilibrium(k, rho, ux, uy);
         const double eo = ps_equilibrium(opp(k), rho, ux, uy);
         const double wr = k <= 4 ? 2 * one18 * 1.0 : one36 * 1.0;
-        fout[k * g.plane + x] = p - (1.0 - b) * (p - eo) * t + b * ((s[k] - ek) - (p - wr));
+        put(k, p - (1.0 - b) * (p - eo) * t + b * ((s[k] - ek) - (p - wr)));
     }
+}
+template <typename T>
+__device__ __forceinline__ void ps_push(const Geometry& g, T* __restrict__ fout, long long node, unsigned bits,
+                                        const double* s, const double* f, double rho, double ux, double uy, double t) {
+    ps_push_values(g, node, bits, s, f, rho, ux, uy, t,
+                   [&](int k, double v) { fout[k * g.plane + node - (DJ(k) * g.ld + DI(k))] = v; });
 }
 
 // One node of a step (steps 1-4 above).  Every lane of the warp calls it

@@ -73,6 +73,17 @@ int stream_box_rows(int storage, int cfg);
 cudaError_t launch_step_stream(int storage, int cfg, const LaunchCtx& ctx, const CUtensorMap* pmap, void* fout,
                                int sm_count);
 
+// Several steps per launch over overlapped register-resident tiles
+// (llb_tile.cuh): at most T steps, halo H rows, TJ columns per block, CPW
+// columns per warp.
+struct TilePlan {
+    int T = 0, H = 0, TJ = 0, CPW = 1;
+};
+bool tile_plan(int storage, int R, int C, bool partial, int sm_count, TilePlan* plan);  // false: one step a launch
+// `steps` plain steps (1..plan.T) from fin to fout; macro: the last one writes rho and u.
+cudaError_t launch_step_tile(int storage, const LaunchCtx& ctx, const TilePlan& plan, const void* fin, void* fout,
+                             int steps, bool macro);
+
 struct BatchLattice;
 // Batched step over a work list (llb_batch.cuh).  `cooperative` launches the
 // grid cooperatively (required when steps > 1).

@@ -269,14 +269,6 @@ struct Rows<ModelShift<__half>, N> : ShiftGroups<__half> {
     }
 };
 
-// 0xff in the byte of every row whose node mask is not active (fluid or open:
-// the two class bits set to 01 or 11, that is bit 0).
-template <class B>
-__device__ __forceinline__ B inactive_rows(B m) {
-    constexpr B one = static_cast<B>(0x0101010101010101ull);
-    return (~m & one) * static_cast<B>(0xff);
-}
-
 // One lane's rows of the node masks or bounce bytes, a byte each.
 template <int RPL>
 struct RowBytes {
@@ -303,13 +295,20 @@ __device__ __forceinline__ constexpr typename RowBytes<RPL>::type each_row(unsig
     return v;
 }
 
+// 0xff in the byte of every row whose node mask is not active (fluid or open:
+// the two class bits 01 or 11, that is bit 0 set).
+template <int RPL, class B>
+__device__ __forceinline__ B inactive_rows(B m) {
+    return (~m & each_row<RPL>(1u)) * static_cast<B>(0xff);
+}
+
 // One column of one warp: f = the populations after step t's collision from s,
 // the pulled ones (bounce-back done), row q of the lane at (i0 + q, j).
-// PLAIN: every row of the warp is a PLAIN fluid node.  mw: the rows' mask
-// bytes.  flag: non-finite densities of this lane's fluid rows are reported in
+// PLAIN: every row of the warp is a PLAIN fluid node.  SOME: the caller knows
+// that at least one row of the lane is active.  mw: the rows' mask bytes.  flag: non-finite densities of this lane's fluid rows are reported in
 // bad.  out(x, rr, xr, yr): the populations, density and velocity of every
 // group, before the collision.
-template <class M, int COLL, bool PLAIN, class P, class B, class Out>
+template <class M, int COLL, bool PLAIN, bool SOME, class P, class B, class Out>
 __device__ __forceinline__ void update_rows(const Geometry& g, const OpenTable& ot, const Collision& c, const P* s,
                                             P* f, B mw, int i0, int j, long long t, bool flag, bool& bad, Out out) {
     using V = typename P::V;
@@ -407,9 +406,11 @@ __device__ __forceinline__ void update_rows(const Geometry& g, const OpenTable& 
         for (int k = 0; k < 9; ++k) f[k].set_group(q, x[q][k]);
     }
     if constexpr (!PLAIN) {
-        const B off = inactive_rows(mw);
+        const B off = inactive_rows<RPL>(mw);
+        if (!SOME || (RPL > 1 && off != 0)) {
 #pragma unroll
-        for (int k = 0; k < 9; ++k) f[k].reset(off, k);
+            for (int k = 0; k < 9; ++k) f[k].reset(off, k);
+        }
     }
 }
 

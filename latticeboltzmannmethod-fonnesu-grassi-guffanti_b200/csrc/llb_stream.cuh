@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(32, CFG::MB)
         if constexpr (sizeof(R) == 8) {
             if (!pl[0]) {  // rows outside the lattice arrive as zeros, not as the initial values
 #pragma unroll
-                for (int k = 0; k < 9; ++k) f[k].reset(inactive_rows(mw[0]), k);
+                for (int k = 0; k < 9; ++k) f[k].reset(inactive_rows<RPL>(mw[0]), k);
             }
         }
 #pragma unroll
@@ -217,11 +217,10 @@ __global__ void __launch_bounds__(32, CFG::MB)
             // columns, once for the others
             const int cc = j - l - 1;
             const auto none = [](const V (*)[9], const V*, const V*, const V*) {};
-            if (pl[l + 1])
-                update_rows<M, COLL, true>(g, ot, c, s, f, mw[l + 1], i0, cc, t0 + l, own_rows, bad, none);
-            else
-                update_rows<M, COLL, false>(g, ot, c, s, f, mw[l + 1], i0, cc, t0 + l,
-                                            own_rows && cc >= c0 && cc < c1, bad, none);
+            // (a non-finite density stays one, so the last level's check finds it)
+            const bool flag = l + 1 == NT && own_rows;
+            if (pl[l + 1]) update_rows<M, COLL, true, false>(g, ot, c, s, f, mw[l + 1], i0, cc, t0 + l, flag, bad, none);
+            else update_rows<M, COLL, false, false>(g, ot, c, s, f, mw[l + 1], i0, cc, t0 + l, flag, bad, none);
             if (l + 1 == NT) {
                 if (own_rows) {
 #pragma unroll

@@ -389,7 +389,8 @@ class CudaLattice:
         0..2 and 6: TMA pipeline configurations (6 also loads the tile's
         bounce bytes); 3..5: two steps per pass, streamed through registers.
         Without this call a large lattice runs its longer runs two steps per
-        pass whatever `pipeline` says of its lone steps."""
+        pass and a small one several steps per launch, whatever `pipeline`
+        says of a lone step."""
         _check(lib().llb_set_pipeline(self._h, config), self._h)
 
     @property
