@@ -31,6 +31,7 @@ SOURCES = {
     "llb_stream.cu": ["--fmad=false"],
     "llb_tile.cu": ["--fmad=false"],
     "llb_capi.cu": [],
+    "llb_copyout.cpp": [],
     "llb_noalloc.cu": [],
     "llb_batch.cu": [],
     "llb_server.cpp": [],

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "../../include/llalbm_cuda.h"
+#include "llb_copyout.h"
 #include "llb_handle.h"
 #include "llb_launch.h"
 
@@ -133,7 +134,7 @@ void release(llb_handle h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (auto& g : h->graph)
         if (g) cudaGraphExecDestroy(g);
-    void* bufs[] = {h->f[0], h->f[1], h->d_mask, h->d_bb, h->d_ps, h->d_psb, h->d_sectors, h->d_smask, h->d_sbb, h->d_open_idx, h->d_open, h->d_rho, h->d_u, h->d_dense,
+    void* bufs[] = {h->f[0], h->f[1], h->d_mask, h->d_bb, h->d_ps, h->d_psb, h->d_sectors, h->d_smask, h->d_sbb, h->d_open_idx, h->d_open, h->d_rho, h->d_dense,
                     h->d_step, h->d_flags, h->d_partials, h->d_red, h->d_fpts, h->d_fdirs, h->d_gather,
                     h->cf[0], h->cf[1], h->d_cnb, h->d_cseg, h->d_cchunk, h->d_ccol, h->d_cinfo};
     for (void* b : bufs) dev_free(h, b);
@@ -143,6 +144,7 @@ void release(llb_handle h) {
         if (e) cudaEventDestroy(e);
     if (h->h_flags) cudaFreeHost(h->h_flags);
     if (h->stream && h->own_stream) cudaStreamDestroy(h->stream);
+    if (h->staging_user) staging_drop_user();
     delete h;
 }
 
@@ -861,11 +863,12 @@ int llb_create(const llb_desc* d, llb_handle* out) {
         (rc = dev_alloc(h, &h->d_mask, mask.size())) || (rc = dev_alloc(h, &h->d_bb, bb.size())) ||
         (rc = dev_alloc(h, &h->d_open_idx, open_idx.size() * sizeof(int32_t))) ||
         (rc = dev_alloc(h, &h->d_open, sizeof(double2) * static_cast<size_t>(std::max<int64_t>(n_open, 1)) * cap)) ||
-        (rc = dev_alloc(h, &h->d_rho, sizeof(double) * N)) || (rc = dev_alloc(h, &h->d_u, sizeof(double) * 2 * N)) ||
+        (rc = dev_alloc(h, &h->d_rho, sizeof(double) * 3 * N)) ||
         (rc = dev_alloc(h, &h->d_step, sizeof(long long))) || (rc = dev_alloc(h, &h->d_flags, sizeof(unsigned))) || (rc = dev_alloc(h, &h->d_red, sizeof(double) * 4)))
         return bail(rc);
     if (!ps.empty() && ((rc = dev_alloc(h, &h->d_ps, ps.size())) || (rc = dev_alloc(h, &h->d_psb, psb.size() * sizeof(double)))))
         return bail(rc);
+    h->d_u = h->d_rho + N;  // rho and u in one buffer: one copy takes both
     e = cudaMemcpyAsync(h->d_mask, mask.data(), mask.size(), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess && h->d_ps)
         e = cudaMemcpyAsync(h->d_ps, ps.data(), ps.size(), cudaMemcpyHostToDevice, h->stream);
@@ -890,6 +893,8 @@ int llb_create(const llb_desc* d, llb_handle* out) {
     h->group_min = default_group_min(*h);
     if (h->group_min == 0 && (h->tma_cfg == PIPE_GRID || h->tma_cfg == PIPE_CLUSTER))
         (void)tile_plan(h->storage, static_cast<int>(h->R), static_cast<int>(h->C), !ps.empty(), h->sm_count, &h->tile);
+    staging_add_user();
+    h->staging_user = true;
     *out = h;
     return LLB_OK;
 }
@@ -997,16 +1002,23 @@ int llb_get_step(llb_handle h, int64_t* step) {
     return LLB_OK;
 }
 
+// rho and u (either may be NULL) from the device to the caller's arrays.
+static int fields_out(llb_handle h, double* rho, double* u) {
+    const size_t bytes = sizeof(double) * static_cast<size_t>(h->R * h->C);
+    HostCopy c[2];
+    int n = 0;
+    if (rho) c[n++] = {rho, h->d_rho, bytes};
+    if (u) c[n++] = {u, h->d_u, 2 * bytes};
+    LLB_CUDA(h, copy_to_host(h->stream, c, n));
+    return LLB_OK;
+}
+
 int llb_get_macro(llb_handle h, double* rho, double* u) {
     if (!h) return fail(nullptr, LLB_E_INVALID, "null handle");
     if (!h->macro_valid) return fail(h, LLB_E_STATE, "no step has written rho/u yet");
     int rc = select_device(h);
     if (rc) return rc;
-    const size_t N = static_cast<size_t>(h->R * h->C);
-    if (rho) LLB_CUDA(h, cudaMemcpyAsync(rho, h->d_rho, sizeof(double) * N, cudaMemcpyDeviceToHost, h->stream));
-    if (u) LLB_CUDA(h, cudaMemcpyAsync(u, h->d_u, sizeof(double) * 2 * N, cudaMemcpyDeviceToHost, h->stream));
-    LLB_CUDA(h, cudaStreamSynchronize(h->stream));
-    return LLB_OK;
+    return fields_out(h, rho, u);
 }
 
 int llb_compute_macro(llb_handle h, double* rho, double* u) {
@@ -1018,11 +1030,7 @@ int llb_compute_macro(llb_handle h, double* rho, double* u) {
     LaunchCtx x = make_ctx(h);
     cudaError_t e = launch_macro_now(h->storage, x, h->f[h->cur], h->step, h->d_rho, h->d_u);
     if (e != cudaSuccess) return cuda_fail(h, e, "macro kernel launch");
-    const size_t N = static_cast<size_t>(h->R * h->C);
-    if (rho) LLB_CUDA(h, cudaMemcpyAsync(rho, h->d_rho, sizeof(double) * N, cudaMemcpyDeviceToHost, h->stream));
-    if (u) LLB_CUDA(h, cudaMemcpyAsync(u, h->d_u, sizeof(double) * 2 * N, cudaMemcpyDeviceToHost, h->stream));
-    LLB_CUDA(h, cudaStreamSynchronize(h->stream));
-    return LLB_OK;
+    return fields_out(h, rho, u);
 }
 
 static int dense_out(llb_handle h, double* host, bool finalize) {
@@ -1037,8 +1045,8 @@ static int dense_out(llb_handle h, double* host, bool finalize) {
     cudaError_t e = finalize ? launch_finalize(h->storage, x, h->f[h->cur], h->d_dense, h->step)
                              : launch_export(h->storage, x, h->f[h->cur], h->d_dense);
     if (e != cudaSuccess) return cuda_fail(h, e, "export kernel launch");
-    LLB_CUDA(h, cudaMemcpyAsync(host, h->d_dense, bytes, cudaMemcpyDeviceToHost, h->stream));
-    LLB_CUDA(h, cudaStreamSynchronize(h->stream));
+    const HostCopy c{host, h->d_dense, bytes};
+    LLB_CUDA(h, copy_to_host(h->stream, &c, 1));
     return LLB_OK;
 }
 
@@ -1080,8 +1088,8 @@ int llb_flow_forces(llb_handle h, double lift_drag[2]) {
     LaunchCtx x = make_ctx(h);
     cudaError_t e = launch_flow_forces(h->storage, x, h->f[h->cur], h->d_fpts, h->d_fdirs, h->n_fpts, h->d_partials, nb, h->d_red);
     if (e != cudaSuccess) return cuda_fail(h, e, "force kernel launch");
-    LLB_CUDA(h, cudaMemcpyAsync(lift_drag, h->d_red, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->stream));
-    LLB_CUDA(h, cudaStreamSynchronize(h->stream));
+    const HostCopy c{lift_drag, h->d_red, sizeof(double) * 2};
+    LLB_CUDA(h, copy_to_host(h->stream, &c, 1));
     return LLB_OK;
 }
 
@@ -1095,8 +1103,8 @@ int llb_gather_force_inputs(llb_handle h, double* values) {
     LaunchCtx x = make_ctx(h);
     cudaError_t e = launch_gather_forces(h->storage, x, h->f[h->cur], h->d_fpts, h->d_fdirs, h->n_fpts, h->d_gather);
     if (e != cudaSuccess) return cuda_fail(h, e, "gather kernel launch");
-    LLB_CUDA(h, cudaMemcpyAsync(values, h->d_gather, sizeof(double) * 8 * h->n_fpts, cudaMemcpyDeviceToHost, h->stream));
-    LLB_CUDA(h, cudaStreamSynchronize(h->stream));
+    const HostCopy c{values, h->d_gather, sizeof(double) * 8 * static_cast<size_t>(h->n_fpts)};
+    LLB_CUDA(h, copy_to_host(h->stream, &c, 1));
     return LLB_OK;
 }
 
@@ -1112,8 +1120,8 @@ int llb_mass_momentum(llb_handle h, double out[3]) {
     LaunchCtx x = make_ctx(h);
     cudaError_t e = launch_mass_momentum(h->storage, x, h->f[h->cur], h->d_partials, nb, h->d_red);
     if (e != cudaSuccess) return cuda_fail(h, e, "reduction kernel launch");
-    LLB_CUDA(h, cudaMemcpyAsync(out, h->d_red, sizeof(double) * 3, cudaMemcpyDeviceToHost, h->stream));
-    LLB_CUDA(h, cudaStreamSynchronize(h->stream));
+    const HostCopy c{out, h->d_red, sizeof(double) * 3};
+    LLB_CUDA(h, copy_to_host(h->stream, &c, 1));
     return LLB_OK;
 }
 

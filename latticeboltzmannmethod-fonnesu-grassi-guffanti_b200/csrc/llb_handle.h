@@ -38,8 +38,9 @@ struct llb_lattice {
     int32_t* d_open_idx = nullptr;
     double2* d_open = nullptr;
     int n_open = 0, cap = 1;
-    double* d_rho = nullptr;
+    double* d_rho = nullptr;  // rho and, behind it, u
     double* d_u = nullptr;
+    bool staging_user = false;  // counted among the users of the host staging buffer
     double* d_dense = nullptr;
     long long* d_step = nullptr;  // step index at the start of a graph replay
     unsigned* d_flags = nullptr;
