@@ -136,7 +136,7 @@ __device__ __forceinline__ void batch_tile(const BatchLattice* __restrict__ Lp, 
         typename M::R rr, xr, yr;
         if (cls == CLS_OPEN) {
             double rho, ux, uy;
-            open_node<M>(Lp->ot, g.open_idx[node], m, t, f, rho, ux, uy);
+            open_node<M>(Lp->ot, open_index(g, node), m, t, f, rho, ux, uy);
             rr = M::from_f64(rho);
             xr = static_cast<typename M::R>(ux);
             yr = static_cast<typename M::R>(uy);
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(BX* BY) k_macro_now(Geometry g, OpenTable ot, 
         typename M::R f[9];
         pull<M>(g, fin, i, j, node, m, false, f);
         if (cls == CLS_OPEN) {
-            open_node<M>(ot, g.open_idx[node], m, t, f, rho, ux, uy);
+            open_node<M>(ot, open_index(g, node), m, t, f, rho, ux, uy);
         } else {
             typename M::R r, x, y;
             M::moments(f, r, x, y);

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1)
         msk[e] = m;
         if (l >= 1 && l <= W) {
             bbs[e - R] = (m & MASK_PLAIN) ? 0u : g.bb[node];
-            oid[e - R] = mask_class(m) == CLS_OPEN ? g.open_idx[node] : -1;
+            oid[e - R] = mask_class(m) == CLS_OPEN ? open_index(g, node) : -1;
         }
 #pragma unroll
         for (int k = 0; k < 9; ++k) {

@@ -167,7 +167,7 @@ __device__ __forceinline__ bool compact_slot(const Geometry& g, const CompactGeo
         typename M::R rr, xr, yr;
         if (cls == CLS_OPEN) {
             double rho, ux, uy;
-            open_node<M>(ot, g.open_idx[nb], m, tstep(), f, rho, ux, uy);
+            open_node<M>(ot, open_index(g, nb), m, tstep(), f, rho, ux, uy);
             rr = M::from_f64(rho);
             xr = static_cast<typename M::R>(ux);
             yr = static_cast<typename M::R>(uy);

@@ -338,7 +338,7 @@ __device__ __forceinline__ void update_rows(const Geometry& g, const OpenTable& 
                     y[k] = P::at(v, q);
                 }
                 double rho, ux, uy;
-                open_node<M>(ot, g.open_idx[static_cast<long long>(j) * g.ld + i0 + q], m, t, y, rho, ux, uy);
+                open_node<M>(ot, open_index(g, static_cast<long long>(j) * g.ld + i0 + q), m, t, y, rho, ux, uy);
 #pragma unroll
                 for (int n = 0; n < NG; ++n)
                     if (n == gq) {

@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(CFG::THREADS, 1)
                         if (si < 0 || sj < 0 || si >= g.rows || sj >= g.cols) f[k] = M::keep(k);
                     }
                     double rho, ux, uy;
-                    open_node<M>(ot, g.open_idx[node], m, current_step(ss), f, rho, ux, uy);
+                    open_node<M>(ot, open_index(g, node), m, current_step(ss), f, rho, ux, uy);
                     rr = M::from_f64(rho);
                     xr = static_cast<R>(ux);
                     yr = static_cast<R>(uy);
