@@ -14,27 +14,39 @@ namespace llb {
 
 namespace {
 
-// Columns of a task.  w: columns each resident warp would walk if the work were
-// spread evenly.  Up to 24: one wave of equal tasks (cavity 1000^2 FP64, w = 16:
-// 17.3 us a step against 19.2 us in tasks of 12 columns and 21.9 us of 24).
-// Above: several waves of smaller tasks, which the block scheduler balances
-// (cavity 4096^2 FP64, w = 256, cj = 28: 212 us against 247 us in one wave and
-// 230 us in tasks of 12 columns, whose four extra columns weigh more).  Edge
-// strips (long path in every column) run chunks half as wide.
+// Columns of a task, four of which it computes or reads besides its own.  w:
+// columns each resident warp would walk if the work were spread evenly.
+// Up to w = 40: the narrowest tasks that are one wave, none left over for a
+// second one.  Against tasks of 12 columns in several waves (us a step): channel
+// 1001 x 3005 FP32, w = 25, 26.4 -> 23.6; cavity 2048^2 FP16, w = 24, 32.1 -> 29.5;
+// porous 1300^2 FP64, w = 27, 31.8 -> 28.8; channel 1500 x 3000 FP32, w = 37, 37.1
+// -> 34.6.  Above, the slowest task of one wave takes too long (cavity 2400^2
+// FP32, w = 46, 48.3 in one wave): several waves, which the block scheduler
+// balances, of sqrt(9 w) columns up to 24 (porous 3600^2 FP32, w = 102, 98.7
+// against 101.9 in tasks of 17 columns; cavity 2900^2 FP32, w = 66, 58.5 against
+// 59.8 in tasks of 14), and of sqrt(3 w) when that is more (cavity 4096^2 FP64, w
+// = 258, 28 columns: 212 against 217 in tasks of 48 and 227 in tasks of 24).
+// Edge strips (long path in every column) run chunks half as wide.
 template <class CFG>
 StreamTasks stream_tasks(int rows, int cols, long long ld, int sm_count) {
     constexpr int EDGE = 2;
     StreamTasks tk{};
     tk.strips = (rows + CFG::V - 1) / CFG::V;
-    const double units = std::max(tk.strips - 2, 0) + EDGE * std::min(tk.strips, 2);
-    const double w = units * cols / (static_cast<double>(sm_count) * CFG::MB);
-    const double cj = w <= 24.0 ? w : std::max(12.0, std::sqrt(3.0 * w));
-    tk.cj = std::min(cols, std::max(4, static_cast<int>(std::ceil(cj))));
+    const int edges = std::min(tk.strips, 2), inner = tk.strips - edges;
+    const long long room = static_cast<long long>(sm_count) * CFG::MB;
+    auto edge_width = [](int c) { return (c + EDGE - 1) / EDGE; };
+    auto chunks = [&](int c) { return (cols + c - 1) / c; };
+    const double w = static_cast<double>(inner + EDGE * edges) * cols / static_cast<double>(room);
+    int cj = std::max(4, static_cast<int>(std::ceil(
+                             w <= 40.0 ? w : std::max(std::min(std::sqrt(9.0 * w), 24.0), std::sqrt(3.0 * w)))));
+    if (w <= 40.0)
+        while (cj < cols && static_cast<long long>(inner) * chunks(cj) + edges * chunks(edge_width(cj)) > room) ++cj;
+    tk.cj = std::min(cols, cj);
     // a task's column offsets are 32-bit byte offsets
     tk.cj = static_cast<int>(std::max(1LL, std::min<long long>(tk.cj, (1LL << 31) / (ld * CFG::ES))));
-    tk.chunks = (cols + tk.cj - 1) / tk.cj;
-    tk.cje = (tk.cj + EDGE - 1) / EDGE;
-    tk.chunks_e = (cols + tk.cje - 1) / tk.cje;
+    tk.chunks = chunks(tk.cj);
+    tk.cje = edge_width(tk.cj);
+    tk.chunks_e = chunks(tk.cje);
     return tk;
 }
 
