@@ -70,12 +70,14 @@ using ModelF16S = ModelShift<__half>;
 // Configurations (eight-byte units per lane, halo rows, stages, warps per SM).
 // The first is the default: 16 warps of 128 registers per SM, 12 of 168 in FP16,
 // whose conversions spill at 128 (cavity 4096^2 FP16: 99 us a step against
-// 124 us).  The second has the other warp count, the third 16 bytes per lane
-// (half the redundant rows, but twice the state: 8 warps per SM).
+// 124 us), and 3 stages (a fourth or fifth takes L1 from the mask bytes: channel
+// 1001 x 3005 FP32 23.4 us a step with 3, 23.8 with 4; FP64 the same).  The second
+// has the other warp count, the third 16 bytes per lane (half the redundant
+// rows, but twice the state: 8 warps per SM).
 template <class M, int H, int MB>
 cudaError_t step_stream(int cfg, const LaunchCtx& x, const CUtensorMap* pm, void* fout, int sm) {
     switch (cfg - FIRST_STREAM_CONFIG) {
-    case 0: return do_step_stream<M, StreamCfg<M, 1, H, 4, MB>>(x, pm, fout, sm);
+    case 0: return do_step_stream<M, StreamCfg<M, 1, H, 3, MB>>(x, pm, fout, sm);
     case 1: return do_step_stream<M, StreamCfg<M, 1, H, 4, 28 - MB>>(x, pm, fout, sm);
     case 2: return do_step_stream<M, StreamCfg<M, 2, H, 4, 8>>(x, pm, fout, sm);
     default: return cudaErrorInvalidValue;
