@@ -167,23 +167,28 @@ inline int default_pipeline(const llb_lattice& h) {
 // Runs of at least this many plain steps take the streaming kernel, two steps
 // per pass (llb_stream.cuh), on lattices whose state no longer sits in L2; 0
 // where they never do.  Measured on B200, us a step, default kernel / streaming:
-//   cavity FP64  724^2 9.3 / 10.3, 850^2 15.5 / 13.0, 1000^2 23.3 / 18.2
-//          FP32  850^2 8.7 / 9.1, 512 x 2048 12.2 / 11.5, 1200^2 18.6 / 15.0
-//          FP16  850^2 9.8 / 10.0, 1000^2 12.7 / 10.8, 2048^2 49.4 / 33.1
+//   cavity FP64  700^2 8.7 / 9.8, 820^2 13.7 / 11.9, 1000^2 23.3 / 17.3; TRT 820^2
+//                14.7 / 15.7, 900^2 18.5 / 17.4, 1024^2 24.5 / 20.3
+//          FP32  820^2 8.3 / 7.7, 900^2 9.6 / 9.4, 1040^2 12.1 / 10.8
+//          FP16  800^2 9.3 / 8.5, 950^2 11.7 / 9.3, 2048^2 49.4 / 29.3
 //   porous (against the compacted planes, which read 30 % fewer nodes)
-//          FP64  1448^2 37.3 / 38.1, 2048^2 70.4 / 67.7, 4096^2 268 / 250
-//          FP32  1024^2 10.0 / 12.7, 1448^2 23.4 / 21.0, 4096^2 162 / 128
-//          FP16  1500 x 2000 26.7 / 27.6, 2048^2 39.9 / 36.6, 4096^2 142 / 119
+//          FP64  BGK 1400^2 36.0 / 32.0, 1700^2 50.1 / 49.3, 2048^2 70.4 / 65.7,
+//                4096^2 268 / 246; TRT, whose arithmetic the compacted planes
+//                hide better, 1774^2 54.8 / 59.7, 2900^2 136 / 142, 4096^2 269 / 284:
+//                never
+//          FP32  1300^2 17.4 / 17.0, 1448^2 23.4 / 19.7, 4096^2 162 / 125
+//          FP16  1800^2 30.1 / 30.6, 2000^2 38.8 / 32.2, 4096^2 142 / 119
 // On the compacted pipeline only longer runs leave its planes: shorter ones
 // would pay for the copies between the layouts.
 inline int default_group_min(const llb_lattice& h) {
     if (h.d_ps || h.n_active == 0) return 0;
     const int64_t n = h.R * h.C;
     const int form = h.storage == LLB_STORE_F64 ? 0 : h.storage == LLB_STORE_F32S ? 1 : 2;
-    static constexpr int64_t kDense[3] = {5LL << 17, 8LL << 17, 7LL << 17};
-    static constexpr int64_t kPorous[3] = {3LL << 20, 2LL << 20, 4LL << 20};
-    if (h.tma_cfg == PIPE_COMPACT) return n >= kPorous[form] ? 32 : 0;
-    return n >= kDense[form] ? llb::STREAM_STEPS : 0;
+    const bool trt64 = form == 0 && h.coll.model == 1;
+    static constexpr int64_t kDense[3] = {5LL << 17, 6LL << 17, 5LL << 17};
+    static constexpr int64_t kPorous[3] = {3LL << 20, 2LL << 20, 7LL << 19};
+    if (h.tma_cfg == PIPE_COMPACT) return n >= kPorous[form] && !trt64 ? 32 : 0;
+    return n >= (trt64 ? 6LL << 17 : kDense[form]) ? llb::STREAM_STEPS : 0;
 }
 
 namespace llb {
