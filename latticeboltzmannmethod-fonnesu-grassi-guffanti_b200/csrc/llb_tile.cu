@@ -26,8 +26,11 @@ cudaError_t do_step_tile(const LaunchCtx& x, const TilePlan& p, const void* fin,
     auto kern = x.c.model == 0 ? k_step_tile<M, 0, CPW, false> : k_step_tile<M, 1, CPW, false>;
     if constexpr (std::is_same_v<M, ModelF64>)
         if (x.g.ps) kern = x.c.model == 0 ? k_step_tile<M, 0, CPW, true> : k_step_tile<M, 1, CPW, true>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // The limit belongs to the kernel, which every handle shares: the most any of
+    // its launches takes, so that what another thread sets is the same.
+    const int most = tile_smem_bytes(TILE_MAX_WARPS, CPW, x.g.ps != nullptr);
+    if (most > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e != cudaSuccess) return e;
     }
     return launch_pdl_smem(kern, grid, block, smem, x.stream, x.g, x.ot, x.c, in, out, x.mo, x.ss, steps, p.H, p.TJ,

@@ -1,0 +1,53 @@
+"""Lattices driven from several host threads: distinct handles are independent."""
+import threading
+
+import numpy as np
+import pytest
+
+import harness as H
+from test_gpu_parity import make_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def saturated(rows, cols):
+    t = H.channel_types(rows, cols, discs=[(rows // 2, cols // 3, 8)])
+    lists = H.classify(t)
+    p = H.Params(tau=0.8, outlet_bc=H.BC_ZH_PRESSURE, obstacle_bc=1, ps_tau=0.8)
+    g = make_gpu(lists, p)
+    v = np.zeros((1, g.n_open, 2))
+    v[0, :len(lists.inlet), 0] = 0.02
+    v[0, len(lists.inlet):, 0] = 1.0
+    g.set_open_values(v)
+    g.init()
+    return g
+
+
+def test_partially_saturated_tiles_of_different_sizes_from_two_threads():
+    """Two lattices whose launches need different amounts of shared memory step
+    at the same time; every call succeeds and both end in the state of a run on
+    one thread."""
+    shapes, calls, per = [(98, 280), (60, 65)], 6000, [3, 5]
+    with saturated(*shapes[0]) as a, saturated(*shapes[1]) as b:
+        errors = []
+
+        def run(g, k):
+            try:
+                for _ in range(calls):
+                    g.step(k)
+                g.synchronize()
+            except Exception as e:  # noqa: BLE001
+                errors.append(e)
+
+        ts = [threading.Thread(target=run, args=x) for x in zip((a, b), per)]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+        assert not errors, errors
+        got = [g.post_collision() for g in (a, b)]
+    for shape, k, post in zip(shapes, per, got):
+        with saturated(*shape) as g:
+            for _ in range(calls):
+                g.step(k)
+            np.testing.assert_array_equal(g.post_collision(), post)
