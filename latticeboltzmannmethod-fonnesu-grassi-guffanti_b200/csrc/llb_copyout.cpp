@@ -13,10 +13,12 @@
 // 12 ms behind queued steps; with the slots 500^2 (6 MB) would take 0.9 ms
 // against 0.39 ms.
 //
-// The small buffer is allocated once per process.  The slots are one
-// process-wide buffer of SLOT x SLOTS bytes, allocated on first use, used
-// by one call at a time (a call that finds it taken copies directly) and freed
-// with the last lattice.
+// Both buffers are the process's, allocated on first use and used by one call at
+// a time: a call that finds one taken copies directly.  The mutex guards who has
+// them and is never held while a call allocates, frees or waits for the GPU, so
+// a lattice is created and destroyed on one thread while another waits for its
+// results.  The small buffer stays for the process, the slots (SLOT x SLOTS
+// bytes) are freed with the last lattice.
 #include "llb_copyout.h"
 
 #include <algorithm>
@@ -38,18 +40,36 @@ constexpr size_t SLOT = size_t{1} << 20;  // bytes of a staging slot
 constexpr size_t SLOTS = 8;
 constexpr size_t MAX_WORKERS = 8;
 
-std::mutex g_mu;  // guards the buffers and is held by the call that uses one
-char* g_small = nullptr;
-char* g_slots = nullptr;
+// A pinned buffer of the process.
+struct Staging {
+    const size_t bytes;
+    char* p = nullptr;
+    bool taken = false;  // a call uses it, or allocates or frees it
+};
+std::mutex g_mu;  // guards the two below and the count of lattices
+Staging g_small{SMALL}, g_slots{SLOT * SLOTS};
 int g_users = 0;
 
-// A pinned buffer, allocated on first use; false if it cannot be had.
-bool reserve(char** p, size_t bytes) {
-    if (*p) return true;
-    if (cudaHostAlloc(reinterpret_cast<void**>(p), bytes, cudaHostAllocPortable) == cudaSuccess) return true;
-    (void)cudaGetLastError();
-    *p = nullptr;
-    return false;
+void give_back(Staging& s) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    s.taken = false;
+}
+
+// The buffer for one call, allocated if it is not there; null if another call
+// has it or no pinned memory can be had.
+char* take(Staging& s) {
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (s.taken) return nullptr;
+        s.taken = true;
+    }
+    if (!s.p && cudaHostAlloc(reinterpret_cast<void**>(&s.p), s.bytes, cudaHostAllocPortable) != cudaSuccess) {
+        (void)cudaGetLastError();
+        s.p = nullptr;
+        give_back(s);
+        return nullptr;
+    }
+    return s.p;
 }
 
 struct Piece {
@@ -73,13 +93,13 @@ cudaError_t direct(cudaStream_t stream, const HostCopy* c, int n) {
     return cudaStreamSynchronize(stream);
 }
 
-cudaError_t small(cudaStream_t stream, const HostCopy* c, int n) {
+cudaError_t small(cudaStream_t stream, const HostCopy* c, int n, char* stage) {
     size_t at = 0;
     for (int q = 0; q < n;) {
         size_t bytes = c[q].bytes;
         int r = q + 1;
         while (r < n && static_cast<const char*>(c[q].src) + bytes == c[r].src) bytes += c[r++].bytes;
-        if (cudaError_t e = cudaMemcpyAsync(g_small + at, c[q].src, bytes, cudaMemcpyDeviceToHost, stream);
+        if (cudaError_t e = cudaMemcpyAsync(stage + at, c[q].src, bytes, cudaMemcpyDeviceToHost, stream);
             e != cudaSuccess)
             return e;
         at += bytes;
@@ -88,7 +108,7 @@ cudaError_t small(cudaStream_t stream, const HostCopy* c, int n) {
     if (cudaError_t e = cudaStreamSynchronize(stream); e != cudaSuccess) return e;
     at = 0;
     for (int q = 0; q < n; ++q) {
-        std::memcpy(c[q].dst, g_small + at, c[q].bytes);
+        std::memcpy(c[q].dst, stage + at, c[q].bytes);
         at += c[q].bytes;
     }
     return cudaSuccess;
@@ -96,13 +116,15 @@ cudaError_t small(cudaStream_t stream, const HostCopy* c, int n) {
 
 // The calling thread feeds the copy engine and waits for it, slot by slot in
 // turn; worker w moves pieces w, w + W, ... on and makes no CUDA call.
-cudaError_t large(cudaStream_t stream, const std::vector<Piece>& pieces, int workers) {
+cudaError_t large(cudaStream_t stream, const std::vector<Piece>& pieces, int workers, char* slots) {
     const size_t n = pieces.size();
     std::atomic<size_t> ready{0};  // pieces in their slots, in order
     std::atomic<bool> stop{false};
     std::unique_ptr<std::atomic<bool>[]> done(new std::atomic<bool>[n]);
     for (size_t q = 0; q < n; ++q) done[q].store(false, std::memory_order_relaxed);
-    auto slot = [](size_t q) { return g_slots + (q % SLOTS) * SLOT; };
+    auto slot = [slots](size_t q) { return slots + (q % SLOTS) * SLOT; };
+    std::vector<std::thread> pool;
+    pool.reserve(static_cast<size_t>(workers));  // (from here on nothing throws out of the call)
     cudaEvent_t ev[SLOTS] = {};
     cudaError_t e = cudaSuccess;
     auto issue = [&](size_t q) {
@@ -125,8 +147,6 @@ cudaError_t large(cudaStream_t stream, const std::vector<Piece>& pieces, int wor
             done[q].store(true, std::memory_order_release);
         }
     };
-    std::vector<std::thread> pool;
-    pool.reserve(static_cast<size_t>(workers));
     int started = 0;
     try {
         for (; started < workers; ++started) pool.emplace_back(work, static_cast<size_t>(started));
@@ -166,36 +186,48 @@ cudaError_t copy_to_host(cudaStream_t stream, const HostCopy* c, int n) {
     size_t total = 0;
     for (int q = 0; q < n; ++q) total += c[q].bytes;
     if (total > SMALL && total < LARGE) return direct(stream, c, n);
-    std::unique_lock<std::mutex> lk(g_mu, std::try_to_lock);
-    if (!lk.owns_lock()) return direct(stream, c, n);
-    if (total <= SMALL) return reserve(&g_small, SMALL) ? small(stream, c, n) : direct(stream, c, n);
+    Staging& stage = total <= SMALL ? g_small : g_slots;
+    char* const buf = take(stage);
+    if (!buf) return direct(stream, c, n);
+    cudaError_t e;
     try {
-        std::vector<Piece> pieces;
-        for (int q = 0; q < n; ++q)
-            for (size_t o = 0; o < c[q].bytes; o += SLOT)
-                pieces.push_back({static_cast<char*>(c[q].dst) + o, static_cast<const char*>(c[q].src) + o,
-                                  std::min(SLOT, c[q].bytes - o)});
-        const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-        const int workers = static_cast<int>(
-            std::min<size_t>({MAX_WORKERS, static_cast<size_t>(hw), pieces.size()}));
-        if (!reserve(&g_slots, SLOT * SLOTS)) return direct(stream, c, n);
-        return large(stream, pieces, workers);
+        if (total <= SMALL) {
+            e = small(stream, c, n, buf);
+        } else {
+            std::vector<Piece> pieces;
+            for (int q = 0; q < n; ++q)
+                for (size_t o = 0; o < c[q].bytes; o += SLOT)
+                    pieces.push_back({static_cast<char*>(c[q].dst) + o, static_cast<const char*>(c[q].src) + o,
+                                      std::min(SLOT, c[q].bytes - o)});
+            const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+            const int workers =
+                static_cast<int>(std::min<size_t>({MAX_WORKERS, static_cast<size_t>(hw), pieces.size()}));
+            e = large(stream, pieces, workers, buf);
+        }
     } catch (const std::bad_alloc&) {
-        return direct(stream, c, n);
+        e = direct(stream, c, n);
     }
+    give_back(stage);
+    return e;
 }
 
 void staging_add_user() {
-    std::lock_guard<std::mutex> lk(g_mu);
-    ++g_users;
-    (void)reserve(&g_small, SMALL);
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        ++g_users;
+    }
+    if (take(g_small)) give_back(g_small);
 }
 
 void staging_drop_user() {
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (--g_users > 0 || !g_slots) return;
-    cudaFreeHost(g_slots);
-    g_slots = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (--g_users > 0 || g_slots.taken || !g_slots.p) return;
+        g_slots.taken = true;
+    }
+    cudaFreeHost(g_slots.p);
+    g_slots.p = nullptr;
+    give_back(g_slots);
 }
 
 }  // namespace llb

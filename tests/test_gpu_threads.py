@@ -1,5 +1,6 @@
 """Lattices driven from several host threads: distinct handles are independent."""
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -51,3 +52,45 @@ def test_partially_saturated_tiles_of_different_sizes_from_two_threads():
             for _ in range(calls):
                 g.step(k)
             np.testing.assert_array_equal(g.post_collision(), post)
+
+
+def cavity(n):
+    import llalbm_cuda as L
+
+    t = np.full((n, n), H.FLUID, dtype=np.uint8)
+    t[0, :] = t[-1, :] = t[:, 0] = t[:, -1] = H.BOUNDARY
+    t[0, 1:-1] = H.INLET
+    g = L.from_types(t, tau=0.8)
+    v = np.zeros((1, g.n_open, 2))
+    v[0, :, 0] = 0.05
+    g.set_open_values(v)
+    g.init()
+    return g
+
+
+def test_lattices_come_and_go_while_another_thread_waits_for_results():
+    """One thread waits for the fields of a lattice with seconds of steps queued;
+    another creates and destroys lattices meanwhile, and is not held up until
+    the results are there."""
+    with cavity(2048) as g:
+        g.step(64, macro=True)
+        g.macro()
+        with cavity(64):
+            pass
+        g.step(20000, macro=True)  # about 1.2 s on the device
+        ready = threading.Event()
+
+        def read():
+            g.macro()
+            ready.set()
+
+        t = threading.Thread(target=read)
+        t.start()
+        time.sleep(0.05)
+        made = 0
+        while made < 3 and not ready.is_set():
+            with cavity(64):
+                pass
+            made += not ready.is_set()
+        t.join()
+        assert made == 3
