@@ -94,3 +94,18 @@ def test_lattices_come_and_go_while_another_thread_waits_for_results():
             made += not ready.is_set()
         t.join()
         assert made == 3
+
+
+def test_waiting_for_results_takes_one_processor():
+    """While a call waits for the steps queued before its results, only the calling
+    thread is busy (it polls an event); the threads that will move the results
+    touch the destination's pages and then sleep."""
+    with cavity(2048) as g:
+        g.step(64, macro=True)
+        g.macro()
+        g.step(20000, macro=True)  # about 1.2 s on the device
+        wall, cpu = time.perf_counter(), time.process_time()
+        g.macro()
+        wall, cpu = time.perf_counter() - wall, time.process_time() - cpu
+    # the copy itself, 100 MB with 9 threads, takes some 5 ms
+    assert wall > 0.3 and cpu < 2.0 * wall
