@@ -8,7 +8,8 @@
 // copy; from LARGE up through pinned slots that worker threads empty -- while
 // the GPU is still at work on the steps queued before, the workers touch the
 // pages of the destination, so the faults are over when the data comes -- and
-// directly in between.  B200 host, rho and u: 48 x 64 43 -> 28 us, 129^2
+// directly in between.  Only ordinary host memory is staged (pageable below).
+// B200 host, rho and u: 48 x 64 43 -> 28 us, 129^2
 // 63 -> 45 us, 2048^2 (101 MB) 22.4 -> 4.7 ms, 4096^2 (403 MB) 86 -> 25 ms, or
 // 12 ms behind queued steps; with the slots 500^2 (6 MB) would take 0.9 ms
 // against 0.39 ms.
@@ -84,6 +85,17 @@ void touch(char* p, size_t bytes) {
         volatile char* q = p + o;
         *q = *q;
     }
+}
+
+// Whether p is ordinary host memory, which the staging is for.  Memory that CUDA
+// knows (pinned, managed, on a device) takes a copy as it is: pinned memory one
+// DMA (2048^2, 101 MB: 1.8 ms, 4.0 through the slots), and a device's memory
+// cannot be written by the host.
+bool pageable(const void* p) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeUnregistered;
+    (void)cudaGetLastError();
+    return false;
 }
 
 cudaError_t direct(cudaStream_t stream, const HostCopy* c, int n) {
@@ -210,6 +222,8 @@ cudaError_t copy_to_host(cudaStream_t stream, const HostCopy* c, int n) {
     size_t total = 0;
     for (int q = 0; q < n; ++q) total += c[q].bytes;
     if (total > SMALL && total < LARGE) return direct(stream, c, n);
+    for (int q = 0; q < n; ++q)
+        if (!pageable(c[q].dst)) return direct(stream, c, n);
     Staging& stage = total <= SMALL ? g_small : g_slots;
     char* const buf = take(stage);
     if (!buf) return direct(stream, c, n);
