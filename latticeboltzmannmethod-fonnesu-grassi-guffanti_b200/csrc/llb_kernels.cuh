@@ -80,37 +80,67 @@ __device__ __forceinline__ long long open_row(const OpenTable& ot, long long t) 
 // population stream (a row of open nodes, a lid, is one warp's chain of
 // dependent loads per column).  Cavity 1000^2 FP64 18.6 -> 17.2 us a step, 2048^2
 // FP32 33.6 -> 32.9.
-__device__ __forceinline__ int open_index(const Geometry& g, long long node) {
+//
+// The kernels of one step make the policy at each load: held through the kernel
+// it takes two registers, and the output steps of the shifted forms 48 instead
+// of 40 (us an output step on 260 x 16000: FP32 80.4 held, 75.4 so; FP16 77.9,
+// 70.3).  The streaming and tile kernels hold one for their masks anyway and
+// pass it (FP16 2048^2 29.2 us a step, 29.6 with a policy at each load).
+struct OwnPolicy {};
+struct HeldPolicy {
+    unsigned long long p;
+};
+__device__ __forceinline__ int open_index(const Geometry& g, long long node, OwnPolicy = {}) {
     int q;
-    asm("ld.global.nc.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(q) : "l"(g.open_idx + node), "l"(l2_keep_policy()));
+    asm("{ .reg .b64 p; createpolicy.fractional.L2::evict_last.b64 p, 1.0;"
+        " ld.global.nc.L2::cache_hint.s32 %0, [%1], p; }"
+        : "=r"(q)
+        : "l"(g.open_idx + node));
     return q;
 }
-__device__ __forceinline__ double2 open_value(const OpenTable& ot, long long t, int q) {
-    const double2* a = ot.vals + open_row(ot, t) * ot.n_open + q;
+__device__ __forceinline__ int open_index(const Geometry& g, long long node, HeldPolicy pol) {
+    int q;
+    asm("ld.global.nc.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(q) : "l"(g.open_idx + node), "l"(pol.p));
+    return q;
+}
+__device__ __forceinline__ const double2* open_slot(const OpenTable& ot, long long t, int q) {
+    return ot.vals + open_row(ot, t) * ot.n_open + q;
+}
+__device__ __forceinline__ double2 open_value(const OpenTable& ot, long long t, int q, OwnPolicy = {}) {
     double2 v;
-    asm("ld.global.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(a), "l"(l2_keep_policy()));
+    asm("{ .reg .b64 p; createpolicy.fractional.L2::evict_last.b64 p, 1.0;"
+        " ld.global.L2::cache_hint.v2.f64 {%0, %1}, [%2], p; }"
+        : "=d"(v.x), "=d"(v.y)
+        : "l"(open_slot(ot, t, q)));
+    return v;
+}
+__device__ __forceinline__ double2 open_value(const OpenTable& ot, long long t, int q, HeldPolicy pol) {
+    double2 v;
+    asm("ld.global.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
+        : "=d"(v.x), "=d"(v.y)
+        : "l"(open_slot(ot, t, q)), "l"(pol.p));
     return v;
 }
 
 // Closure + choice of (rho, u) for an open node at step t (t >= 1), or for the
 // initial step (t == 0: no closure, pressure nodes start at rest).
-template <class M>
+template <class M, class Pol = OwnPolicy>
 __device__ __forceinline__ void open_node(const OpenTable& ot, int q, uint8_t m, long long t, typename M::R* f,
-                                          double& rho, double& ux, double& uy) {
+                                          double& rho, double& ux, double& uy, Pol pol = {}) {
     const int side = mask_side(m), bc = mask_bc(m);
-    const double2 cur = open_value(ot, t, q);
+    const double2 cur = open_value(ot, t, q, pol);
     if (bc == BC_ZH_PRES) {
         rho = cur.x;
         if (t == 0) {
             ux = 0.0;
             uy = 0.0;
         } else {
-            const double2 prev = open_value(ot, t - 1, q);
+            const double2 prev = open_value(ot, t - 1, q, pol);
             M::closure_pressure(f, side, prev.x, prev.y, ux, uy);
         }
     } else {
         if (bc == BC_ZH_VEL && t > 0) {
-            const double2 prev = open_value(ot, t - 1, q);
+            const double2 prev = open_value(ot, t - 1, q, pol);
             M::closure_velocity(f, side, prev.x, prev.y);
         }
         rho = 1.0;  // open nodes collide with global_rho == 1 (never written for them)

@@ -305,12 +305,14 @@ __device__ __forceinline__ B inactive_rows(B m) {
 // One column of one warp: f = the populations after step t's collision from s,
 // the pulled ones (bounce-back done), row q of the lane at (i0 + q, j).
 // PLAIN: every row of the warp is a PLAIN fluid node.  SOME: the caller knows
-// that at least one row of the lane is active.  mw: the rows' mask bytes.  flag: non-finite densities of this lane's fluid rows are reported in
-// bad.  out(x, rr, xr, yr): the populations, density and velocity of every
-// group, before the collision.
+// that at least one row of the lane is active.  mw: the rows' mask bytes.  pol:
+// the policy of the open nodes' table reads.  flag: non-finite densities of this
+// lane's fluid rows are reported in bad.  out(x, rr, xr, yr): the populations,
+// density and velocity of every group, before the collision.
 template <class M, int COLL, bool PLAIN, bool SOME, class P, class B, class Out>
 __device__ __forceinline__ void update_rows(const Geometry& g, const OpenTable& ot, const Collision& c, const P* s,
-                                            P* f, B mw, int i0, int j, long long t, bool flag, bool& bad, Out out) {
+                                            P* f, B mw, int i0, int j, long long t, HeldPolicy pol, bool flag,
+                                            bool& bad, Out out) {
     using V = typename P::V;
     using R = typename M::R;
     constexpr int NG = P::NG, RG = P::RG, RPL = P::RPL;
@@ -338,7 +340,8 @@ __device__ __forceinline__ void update_rows(const Geometry& g, const OpenTable& 
                     y[k] = P::at(v, q);
                 }
                 double rho, ux, uy;
-                open_node<M>(ot, open_index(g, static_cast<long long>(j) * g.ld + i0 + q), m, t, y, rho, ux, uy);
+                open_node<M>(ot, open_index(g, static_cast<long long>(j) * g.ld + i0 + q, pol), m, t, y, rho, ux, uy,
+                             pol);
 #pragma unroll
                 for (int n = 0; n < NG; ++n)
                     if (n == gq) {

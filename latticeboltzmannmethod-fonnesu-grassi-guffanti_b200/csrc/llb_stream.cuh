@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(32, CFG::MB)
     const bool row_in = i0 >= 0 && i0 < g.ld;
     const bool own_rows = lane >= H / RPL && lane < 32 - H / RPL && i0 < g.rows;
     const unsigned long long pol = l2_keep_policy();
+    const HeldPolicy held{pol};
     B nm = 0, nb = 0;  // masks and bounce bytes of the next column
     auto fetch_bytes = [&](int j) {
         nm = 0;
@@ -219,8 +220,8 @@ __global__ void __launch_bounds__(32, CFG::MB)
             const auto none = [](const V (*)[9], const V*, const V*, const V*) {};
             // (a non-finite density stays one, so the last level's check finds it)
             const bool flag = l + 1 == NT && own_rows;
-            if (pl[l + 1]) update_rows<M, COLL, true, false>(g, ot, c, s, f, mw[l + 1], i0, cc, t0 + l, flag, bad, none);
-            else update_rows<M, COLL, false, false>(g, ot, c, s, f, mw[l + 1], i0, cc, t0 + l, flag, bad, none);
+            if (pl[l + 1]) update_rows<M, COLL, true, false>(g, ot, c, s, f, mw[l + 1], i0, cc, t0 + l, held, flag, bad, none);
+            else update_rows<M, COLL, false, false>(g, ot, c, s, f, mw[l + 1], i0, cc, t0 + l, held, flag, bad, none);
             if (l + 1 == NT) {
                 if (own_rows) {
 #pragma unroll

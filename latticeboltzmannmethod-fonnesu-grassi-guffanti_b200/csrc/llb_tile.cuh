@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(32 * TILE_MAX_WARPS)
     [[maybe_unused]] unsigned pw[CPW];
     bool pl[CPW];
     const unsigned long long pol = l2_keep_policy();
+    const HeldPolicy held{pol};
 #pragma unroll
     for (int q = 0; q < CPW; ++q) {
         const int j = j0 + q;
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(32 * TILE_MAX_WARPS)
                     });
                 };
                 if (pl[q]) {
-                    update_rows<M, COLL, true, true>(g, ot, c, s9, f[q], mw[q], i0, j, t0 + s, mine, bad, out);
+                    update_rows<M, COLL, true, true>(g, ot, c, s9, f[q], mw[q], i0, j, t0 + s, held, mine, bad, out);
                 } else if (inactive_rows<RPL>(mw[q]) == each_row<RPL>(0xffu)) {
                     fields([](int, int) { return 0.0; });  // no active row: f keeps the initial values
                 } else {
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(32 * TILE_MAX_WARPS)
                         for (int k = 1; k < 9; ++k)
                             if ((pw[q] >> (k - 1)) & 1u) s9[k].v[0] = v[(k - 1) * 32];
                         double sp[9], prr = 0.0, pxr = 0.0, pyr = 0.0;
-                        update_rows<M, COLL, false, true>(g, ot, c, s9, f[q], mw[q], i0, j, t0 + s, mine, bad,
+                        update_rows<M, COLL, false, true>(g, ot, c, s9, f[q], mw[q], i0, j, t0 + s, held, mine, bad,
                                                     [&](const V (*x)[9], const V* rr, const V* xr, const V* yr) {
                                                         out(x, rr, xr, yr);
 #pragma unroll
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(32 * TILE_MAX_WARPS)
                                 ps_push(g, fout, node, pw[q], sp, fp, prr, pxr, pyr, c.ps_t);
                         }
                     } else {
-                        update_rows<M, COLL, false, true>(g, ot, c, s9, f[q], mw[q], i0, j, t0 + s, mine, bad, out);
+                        update_rows<M, COLL, false, true>(g, ot, c, s9, f[q], mw[q], i0, j, t0 + s, held, mine, bad, out);
                     }
                 }
                 if (mine) {
