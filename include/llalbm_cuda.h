@@ -428,10 +428,27 @@ int llb_event_elapsed_ms(llb_handle h, int32_t slot_begin, int32_t slot_end, flo
    configurations compute the same per-node arithmetic and give the same bits
    in every storage form. */
 int llb_set_pipeline(llb_handle h, int32_t config);
+/* The configuration in use.  A lattice whose configuration was never set may
+   step its runs another way than a lone step: large ones two steps per pass,
+   small ones several steps per launch in tiles that sit in registers.
+   llb_get_pipeline then reports the configuration of a lone step,
+   llb_run_kernel what a given run takes.  llb_set_pipeline makes every step of
+   the lattice run on the configuration it names, the one reported included;
+   llb_reset_pipeline goes back to the way the lattice was created with. */
 int llb_get_pipeline(llb_handle h, int32_t* config);
+int llb_reset_pipeline(llb_handle h);
+/* Which kernel the plain steps of llb_step(h, nsteps, flags) run on (the output
+   step, when it is the only one): a configuration as above, or LLB_KERNEL_TILES,
+   and the steps one launch of it advances.  No reference counterpart. */
+#define LLB_KERNEL_TILES 16 /* several steps per launch in register-resident tiles */
+int llb_run_kernel(llb_handle h, int32_t nsteps, uint32_t flags, int32_t* config, int32_t* steps_per_launch);
 /* Autotuner of one lattice (no reference counterpart): runs every plain-step
    configuration this lattice supports (-4..-1, 0..6) for trial_steps warm-up
-   and trial_steps timed steps and keeps the fastest.  Every configuration
+   and trial_steps timed steps and keeps the fastest.  The default configuration
+   of a lattice that steps in tiles by default is tried both ways, in tiles and
+   without, for half of these steps each; if the tiles win, best is that
+   configuration and the lattice steps in tiles (llb_run_kernel tells), as
+   another lattice like it does from creation on.  Every configuration
    gives the same bits, so these are ordinary steps of the simulation: the
    lattice advances by 2 x trial_steps per configuration tried (llb_get_step
    tells how far), and their boundary values must be set as for llb_step.

@@ -351,8 +351,25 @@ int run_config(llb_handle h, int32_t plain) {
     return h->group_min > 0 && plain >= h->group_min ? FIRST_STREAM_CONFIG : h->tma_cfg;
 }
 
+// Whether llb_step of `nsteps` steps, the last of them an output step if
+// `macro`, runs in tiles.
+bool run_in_tiles(llb_handle h, int32_t, bool) { return h->tile.T > 0; }
+
+// The lattice's default way of stepping, kept beside the configuration in use.
+void keep_default(llb_handle h) {
+    h->def_cfg = h->tma_cfg;
+    h->def_group_min = h->group_min;
+    h->def_tile = h->tile;
+}
+
 // Steps one plain-step launch of a configuration advances.
 int steps_per_launch(int cfg) { return is_stream(cfg) ? STREAM_STEPS : 1; }
+
+// The kernel of a lone step left over by a two-step configuration: the handle's
+// own dense kernel, else one thread per node.
+int lone_config(llb_handle h) {
+    return is_stream(h->tma_cfg) || h->tma_cfg == PIPE_COMPACT ? PIPE_GRID : h->tma_cfg;
+}
 
 // ---------------------------------------------------------------------------
 // column-compacted storage (pipeline PIPE_COMPACT)
@@ -598,14 +615,20 @@ int launch_one(llb_handle h, int cfg, bool macro, long long graph_offset = -1) {
     return LLB_OK;
 }
 
-// nsteps steps of a lattice that steps in tiles, several per launch, evenly
-// split; with macro the last one writes rho and u.
+// Steps of the next launch of a lattice that steps in tiles, `left` to go:
+// evenly split.
+int32_t tile_steps(llb_handle h, int32_t left) {
+    const int32_t launches = (left + h->tile.T - 1) / h->tile.T;
+    return (left + launches - 1) / launches;
+}
+
+// nsteps steps of a lattice that steps in tiles; with macro the last one writes
+// rho and u.
 int step_tiles(llb_handle h, int32_t nsteps, bool macro) {
     int rc = state_to_dense(h);
     if (rc) return rc;
     for (int32_t left = nsteps; left > 0;) {
-        const int32_t launches = (left + h->tile.T - 1) / h->tile.T;
-        const int32_t k = (left + launches - 1) / launches;
+        const int32_t k = tile_steps(h, left);
         const bool out = macro && k == left;
         cudaError_t e = launch_step_tile(h->storage, make_ctx(h), h->tile, h->f[h->cur], h->f[h->cur ^ 1], k, out);
         if (e != cudaSuccess) return cuda_fail(h, e, "tile step kernel launch");
@@ -752,6 +775,7 @@ int handle_leave_compact(llb_handle h) {
     h->tma_cfg = default_dense_pipeline(*h);
     h->maps_ready = false;
     release_compact(h);
+    if (h->def_cfg == PIPE_COMPACT) h->def_cfg = h->tma_cfg;
     return LLB_OK;
 }
 }  // namespace llb
@@ -893,6 +917,7 @@ int llb_create(const llb_desc* d, llb_handle* out) {
     h->group_min = default_group_min(*h);
     if (h->group_min == 0 && (h->tma_cfg == PIPE_GRID || h->tma_cfg == PIPE_CLUSTER))
         (void)tile_plan(h->storage, static_cast<int>(h->R), static_cast<int>(h->C), !ps.empty(), h->sm_count, &h->tile);
+    keep_default(h);
     staging_add_user();
     h->staging_user = true;
     *out = h;
@@ -949,7 +974,7 @@ int llb_step(llb_handle h, int32_t nsteps, uint32_t flags) {
     int rc = select_device(h);
     if (rc) return rc;
     const bool macro = (flags & LLB_STEP_MACRO) != 0;
-    if (h->tile.T > 0) return step_tiles(h, nsteps, macro);
+    if (run_in_tiles(h, nsteps, macro)) return step_tiles(h, nsteps, macro);
     int32_t plain = macro ? nsteps - 1 : nsteps;
     const int cfg = run_config(h, plain);
     const bool compact = cfg == PIPE_COMPACT;
@@ -981,11 +1006,8 @@ int llb_step(llb_handle h, int32_t nsteps, uint32_t flags) {
     const int per = steps_per_launch(cfg);
     for (; plain >= per; plain -= per)
         if ((rc = launch_one(h, cfg, false))) return rc;
-    // a lone step left over by a two-step configuration: the handle's own dense
-    // kernel, else one thread per node
-    const int lone = is_stream(h->tma_cfg) || h->tma_cfg == PIPE_COMPACT ? PIPE_GRID : h->tma_cfg;
-    for (; plain > 0; --plain)
-        if ((rc = launch_one(h, lone, false))) return rc;
+    for (; plain > 0; --plain)  // a lone step left over by a two-step configuration
+        if ((rc = launch_one(h, lone_config(h), false))) return rc;
     if (macro) {
         // output steps write rho and u from the dense kernel
         if ((rc = state_to_dense(h))) return rc;
@@ -1252,6 +1274,14 @@ static int build_sector_list(llb_handle h) {
     return LLB_OK;
 }
 
+// Waits for the handle's stream and destroys its graphs.
+static int drop_graphs(llb_handle h) {
+    LLB_CUDA(h, cudaStreamSynchronize(h->stream));
+    for (auto& g : h->graph)
+        if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+    return LLB_OK;
+}
+
 int llb_set_pipeline(llb_handle h, int32_t config) {
     if (!h || config < PIPE_CLUSTER || config >= TMA_CONFIGS)
         return fail(h, LLB_E_INVALID, "config must be -4, -3, -2, -1 or in [0, 7)");
@@ -1271,15 +1301,43 @@ int llb_set_pipeline(llb_handle h, int32_t config) {
         if (config == PIPE_LIST && (rc = build_sector_list(h))) return rc;
         if (config == PIPE_COMPACT && (rc = build_compact(h))) return rc;
         if (h->tma_cfg == PIPE_COMPACT && (rc = state_to_dense(h))) return rc;
-        LLB_CUDA(h, cudaStreamSynchronize(h->stream));
-        for (auto& g : h->graph)
-            if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+        if ((rc = drop_graphs(h))) return rc;
         h->tma_cfg = config;
         h->group_min = 0;
         h->tile = TilePlan{};
         h->maps_ready = false;
-
     }
+    return LLB_OK;
+}
+
+int llb_reset_pipeline(llb_handle h) {
+    if (!h) return fail(nullptr, LLB_E_INVALID, "null handle");
+    if (h->tma_cfg == h->def_cfg && h->group_min == h->def_group_min && h->tile.T == h->def_tile.T) return LLB_OK;
+    if (int rc = llb_set_pipeline(h, h->def_cfg)) return rc;
+    if (int rc = drop_graphs(h)) return rc;  // of the same configuration without its longer runs' kernel
+    h->group_min = h->def_group_min;
+    h->tile = h->def_tile;
+    return LLB_OK;
+}
+
+int llb_run_kernel(llb_handle h, int32_t nsteps, uint32_t flags, int32_t* config, int32_t* per_launch) {
+    if (!h || nsteps < 1 || !config || !per_launch) return fail(h, LLB_E_INVALID, "bad arguments");
+    const bool macro = (flags & LLB_STEP_MACRO) != 0;
+    if (run_in_tiles(h, nsteps, macro)) {
+        *config = LLB_KERNEL_TILES;
+        *per_launch = tile_steps(h, nsteps);
+        return LLB_OK;
+    }
+    const int32_t plain = macro ? nsteps - 1 : nsteps;
+    if (plain == 0) {  // an output step alone: the one-thread kernel
+        *config = PIPE_GRID;
+        *per_launch = 1;
+        return LLB_OK;
+    }
+    int cfg = run_config(h, plain);
+    if (plain < steps_per_launch(cfg)) cfg = lone_config(h);
+    *config = cfg;
+    *per_launch = cfg == PIPE_CLUSTER ? std::min<int32_t>(plain, CLUSTER_CHUNK) : steps_per_launch(cfg);
     return LLB_OK;
 }
 
@@ -1317,49 +1375,53 @@ int llb_tune_pipeline(llb_handle h, int32_t trial_steps, int32_t* best, float* m
         cudaEventDestroy(e0);
         return cuda_fail(h, ce, "cudaEventCreate");
     }
-    // the configuration the handle came with is timed as it steps by default
-    const int original = h->tma_cfg, group_min = h->group_min;
-    const TilePlan tile = h->tile;
-    auto by_default = [&] {
-        h->group_min = group_min;
-        h->tile = tile;
+    // A lattice that steps in tiles by default: its configuration is timed both
+    // ways, each for half of the steps.  (A lattice whose longer runs stream by
+    // default needs no more than the list: configuration 3 is how they run.)
+    const bool tiles = h->def_tile.T > 0;
+    int chosen = h->tma_cfg;
+    bool chosen_tiles = false;
+    float chosen_ms = -1.0f;  // per step
+    // n warm-up steps (tensor maps, graphs), then n timed steps
+    auto timed = [&](int32_t n, float* ms) -> int {
+        if (int r = llb_step(h, n, 0)) return r;
+        cudaError_t te = cudaEventRecord(e0, h->stream);
+        if (te != cudaSuccess) return cuda_fail(h, te, "cudaEventRecord");
+        if (int r = llb_step(h, n, 0)) return r;
+        te = cudaEventRecord(e1, h->stream);
+        if (te == cudaSuccess) te = cudaEventSynchronize(e1);
+        if (te == cudaSuccess) te = cudaEventElapsedTime(ms, e0, e1);
+        if (te != cudaSuccess) return cuda_fail(h, te, "timing a pipeline configuration");
+        *ms /= static_cast<float>(n);
+        return LLB_OK;
     };
-    int chosen = original;
-    float chosen_ms = -1.0f;
     static constexpr int kCandidates[] = {PIPE_GRID, PIPE_LIST, PIPE_COMPACT, PIPE_CLUSTER, 0, 1, 2, 3, 4, 5, 6};
     for (int cfg : kCandidates) {
         if (llb_set_pipeline(h, cfg) != LLB_OK) continue;  // not available for this lattice
-        if (cfg == original) by_default();
-        // warm-up (tensor maps, graphs), then the timed steps
-        if ((rc = llb_step(h, trial_steps, 0))) break;
-        cudaError_t te = cudaEventRecord(e0, h->stream);
-        if (te != cudaSuccess) {
-            rc = cuda_fail(h, te, "cudaEventRecord");
-            break;
+        const bool both = tiles && cfg == h->def_cfg;
+        const int32_t n_tiles = both ? trial_steps / 2 : 0;
+        for (bool in_tiles : {false, true}) {
+            if (in_tiles && !both) break;
+            if (in_tiles) h->tile = h->def_tile;
+            float ms = 0.0f;
+            if ((rc = timed(in_tiles ? n_tiles : trial_steps - n_tiles, &ms))) break;
+            if (chosen_ms < 0.0f || ms < chosen_ms) {
+                chosen_ms = ms;
+                chosen = cfg;
+                chosen_tiles = in_tiles;
+            }
         }
-        if ((rc = llb_step(h, trial_steps, 0))) break;
-        float ms = 0.0f;
-        te = cudaEventRecord(e1, h->stream);
-        if (te == cudaSuccess) te = cudaEventSynchronize(e1);
-        if (te == cudaSuccess) te = cudaEventElapsedTime(&ms, e0, e1);
-        if (te != cudaSuccess) {
-            rc = cuda_fail(h, te, "timing a pipeline configuration");
-            break;
-        }
-        if (chosen_ms < 0.0f || ms < chosen_ms) {
-            chosen_ms = ms;
-            chosen = cfg;
-        }
+        if (rc) break;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (rc) return rc;
     if ((rc = llb_set_pipeline(h, chosen))) return rc;
-    if (chosen == original) by_default();
+    if (chosen_tiles) h->tile = h->def_tile;
     if (chosen != PIPE_LIST) release_sector_list(h);
     if (chosen != PIPE_COMPACT) release_compact(h);
     if (best) *best = chosen;
-    if (ms_per_step) *ms_per_step = chosen_ms < 0.0f ? 0.0f : chosen_ms / static_cast<float>(trial_steps);
+    if (ms_per_step) *ms_per_step = chosen_ms < 0.0f ? 0.0f : chosen_ms;
     return LLB_OK;
 }
 

@@ -110,6 +110,10 @@ struct llb_lattice {
     // T == 0: off): the plain and output steps of a lattice that fits L2 on its
     // default kernel.  llb_set_pipeline turns it off.
     llb::TilePlan tile;
+    // the way of stepping the lattice was created with (llb_reset_pipeline)
+    int def_cfg = -1;
+    int def_group_min = 0;
+    llb::TilePlan def_tile;
 };
 
 // Residence of the state (llb_lattice::where).  Steps of the compacted

@@ -30,6 +30,7 @@ PATTERN_AB, PATTERN_AA = 0, 1
 BC_ZH_VELOCITY, BC_OPEN, BC_ZH_PRESSURE = 0, 1, 2
 OBSTACLE_BOUNCE_BACK, OBSTACLE_PARTIAL = 0, 1
 STEP_MACRO = 1
+KERNEL_TILES = 16  # run_kernel: several steps per launch in register-resident tiles
 SERVE_BATCHED, SERVE_SEQUENTIAL = 0, 1
 ADMIT_SHORTEST_FIRST, ADMIT_FIFO = 0, 1
 LAYOUT_AUTO, LAYOUT_COMPACT, LAYOUT_DENSE = 0, 1, 2
@@ -101,6 +102,9 @@ SIGNATURES = {
     "llb_event_elapsed_ms": [_H, ctypes.c_int32, ctypes.c_int32, ctypes.POINTER(ctypes.c_float)],
     "llb_set_pipeline": [_H, ctypes.c_int32],
     "llb_get_pipeline": [_H, ctypes.POINTER(ctypes.c_int32)],
+    "llb_reset_pipeline": [_H],
+    "llb_run_kernel": [_H, ctypes.c_int32, ctypes.c_uint32, ctypes.POINTER(ctypes.c_int32),
+                       ctypes.POINTER(ctypes.c_int32)],
     "llb_tune_pipeline": [_H, ctypes.c_int32, ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_float)],
     "llb_set_launch_shape": [_H, ctypes.c_int32],
     "llb_set_wait_limit": [_H, ctypes.c_int64],
@@ -390,8 +394,21 @@ class CudaLattice:
         bounce bytes); 3..5: two steps per pass, streamed through registers.
         Without this call a large lattice runs its longer runs two steps per
         pass and a small one several steps per launch, whatever `pipeline`
-        says of a lone step."""
+        says of a lone step (run_kernel tells); reset_pipeline goes back to
+        that."""
         _check(lib().llb_set_pipeline(self._h, config), self._h)
+
+    def reset_pipeline(self):
+        """Back to the way of stepping the lattice was created with."""
+        _check(lib().llb_reset_pipeline(self._h), self._h)
+
+    def run_kernel(self, n: int, macro: bool = False):
+        """Kernel of the plain steps of step(n, macro) -- a configuration of
+        set_pipeline or KERNEL_TILES -- and the steps one launch advances."""
+        c, per = ctypes.c_int32(), ctypes.c_int32()
+        _check(lib().llb_run_kernel(self._h, n, STEP_MACRO if macro else 0, ctypes.byref(c), ctypes.byref(per)),
+               self._h)
+        return c.value, per.value
 
     @property
     def pipeline(self) -> int:
