@@ -916,7 +916,8 @@ int llb_create(const llb_desc* d, llb_handle* out) {
     }
     h->group_min = default_group_min(*h);
     if (h->group_min == 0 && (h->tma_cfg == PIPE_GRID || h->tma_cfg == PIPE_CLUSTER))
-        (void)tile_plan(h->storage, static_cast<int>(h->R), static_cast<int>(h->C), !ps.empty(), h->sm_count, &h->tile);
+        (void)tile_plan(h->storage, static_cast<int>(h->R), static_cast<int>(h->C), !ps.empty(),
+                        h->tma_cfg == PIPE_CLUSTER, h->sm_count, &h->tile);
     keep_default(h);
     staging_add_user();
     h->staging_user = true;

@@ -79,7 +79,9 @@ cudaError_t launch_step_stream(int storage, int cfg, const LaunchCtx& ctx, const
 struct TilePlan {
     int T = 0, H = 0, TJ = 0, CPW = 1;
 };
-bool tile_plan(int storage, int R, int C, bool partial, int sm_count, TilePlan* plan);  // false: one step a launch
+// False: one step a launch.  cluster: the lattice's one-step default is the
+// cluster kernel.
+bool tile_plan(int storage, int R, int C, bool partial, bool cluster, int sm_count, TilePlan* plan);
 // `steps` plain steps (1..plan.T) from fin to fout; macro: the last one writes rho and u.
 cudaError_t launch_step_tile(int storage, const LaunchCtx& ctx, const TilePlan& plan, const void* fin, void* fout,
                              int steps, bool macro);

@@ -48,41 +48,49 @@ cudaError_t step_tile(const LaunchCtx& x, const TilePlan& p, const void* fin, vo
 
 }  // namespace
 
-// The shape whose launches cost least per step: a launch's fixed cost, the load
-// of a tile, and per step the larger of one warp's chain over its columns and
-// the columns an SM updates (0.05 us a column in every form: about 200
-// instructions on one of four schedulers).  The model chose, out of every
-// shape measured on 31 lattices x forms (40^2 to 500 x 800), one within 9 % of
-// the best and 1.2 % of it on average.
+// The shape whose launches cost least per step, among those with a tile per SM
+// at most: a launch's fixed cost and the load of a tile, and per step the larger
+// of one warp's chain over its columns and the columns a tile updates (0.05 us a
+// column in every form: about 200 instructions on one of four schedulers).  The
+// model ranks shapes and no more (129^2 FP64: 0.85 us by it, 1.5 measured); out
+// of every shape measured on 31 lattices x forms it chose one within 9 % of the
+// best and 1.2 % of it on average.
 //
-// Lattices in the range below gain; us a step on B200, default kernel before /
-// tiles: FP64 64^2 1.93 / 1.34, 129^2 3.08 / 1.57, 150 x 600 4.17 / 2.85, but
-// 300 x 500 4.30 / 4.37; FP32 129^2 2.94 / 1.66, 300 x 500 4.28 / 2.77, but
-// 500^2 4.79 / 6.5; FP16 64^2 1.82 / 2.00 (the cluster kernel), 129^2
-// 2.96 / 1.97, 256 x 1024 6.19 / 4.72, 500 x 800 7.51 / 7.28; partially
-// saturated obstacles 100 x 250 3.28 / 2.14, but 150 x 600 3.81 / 4.28.
-bool tile_plan(int storage, int R, int C, bool partial, int sm_count, TilePlan* plan) {
+// With no more tiles than SMs every block starts at once.  With two or more per
+// SM the second wave's launch ends long after the first's, and whether tiles win
+// is chance: us a step, one-step kernels / tiles, FP64 256 x 400 4.40 / 4.68, TRT
+// 4.43 / 5.14, 300 x 380 4.26 / 4.70, TRT 4.30 / 5.29, 3 x 30000 26.4 / 28.3;
+// FP32 400 x 490 4.40 / 4.96, 16 x 12000 10.2 / 14.2; FP16 10 x 4000 6.9 / 9.0,
+// 130 x 3000 8.9 / 9.9, 7 x 13053 11.5 / 25.2 (and some gain: FP64 16 x 7000
+// 7.76 / 5.86, FP32 channel 400 x 490 4.62 / 4.20).
+//
+// One wave, us a step, one-step kernels / tiles: FP64 64^2 1.93 / 1.34, 129^2
+// 3.22 / 1.52, 181 x 333 3.72 / 3.04, TRT 3.73 / 3.32, 1492 x 43 TRT 3.28 / 2.99;
+// FP32 129^2 3.09 / 1.62, 256 x 400 3.97 / 3.02, 440 x 450 4.40 / 3.95; FP16 64^2
+// 1.82 / 2.00 (the cluster kernel), 129^2 3.27 / 1.90, 256 x 1024 6.06 / 5.13,
+// 680 x 578 6.92 / 5.94.  Two columns a warp are not taken with partially
+// saturated obstacles (100 x 250, one column, 3.33 / 2.10; 200 x 249, two, 3.42 /
+// 3.60, TRT 3.44 / 3.82) and not against the cluster kernel, whose lattices need
+// them only when they are a few rows high, most of a tile outside (3 x 3900 FP64
+// 2.1 / 4.1, FP32 1.9 / 5.0; 8 x 3000 FP16 1.17 times the cluster's).
+bool tile_plan(int storage, int R, int C, bool partial, bool cluster, int sm_count, TilePlan* plan) {
     *plan = TilePlan{};
     const int form = partial ? 3 : storage == LLB_STORE_F64 ? 0 : storage == LLB_STORE_F32S ? 1 : 2;
     static constexpr long long kMost[4] = {115000, 200000, 400000, 50000}, kLeast[4] = {0, 0, 8000, 0};
     const long long nodes = static_cast<long long>(R) * C;
     if (nodes > kMost[form] || nodes < kLeast[form]) return false;
     const int rpl = form == 1 ? 2 : form == 2 ? 4 : 1;
-    // registers per thread of the kernels (columns per warp 1, 2)
-    static constexpr int kRegs[4][2] = {{84, 126}, {120, 104}, {126, 128}, {128, 128}};
+    const int most_cpw = partial || cluster ? 1 : 2;
     double best = 1e30;
     for (int T : {3, 4, 5, 6, 8})
-        for (int cpw : {1, 2})
+        for (int cpw = 1; cpw <= most_cpw; ++cpw)
             for (int nw = 8; nw <= 16; nw += 2) {
                 const int H = (T + rpl - 1) / rpl * rpl, V = 32 * rpl - 2 * H, TJ = nw * cpw - 2 * T;
                 if (TJ < 2) continue;
                 const long long tiles = static_cast<long long>((R + V - 1) / V) * ((C + TJ - 1) / TJ);
-                const int resident = std::max(1, std::min(64 / nw, 65536 / (kRegs[form][cpw - 1] * 32 * nw)));
-                const long long per_sm = (tiles + sm_count - 1) / sm_count;
-                const double waves = static_cast<double>((per_sm + resident - 1) / resident);
-                const double columns = static_cast<double>(std::min<long long>(per_sm, resident)) * (nw * cpw - T);
-                const double step = std::max(0.1 + 0.4 * cpw, 0.05 * columns);
-                const double t = (1.2 + waves * (0.3 + T * step)) / T;
+                if (tiles > sm_count) continue;
+                const double step = std::max(0.1 + 0.4 * cpw, 0.05 * (nw * cpw - T));
+                const double t = (1.5 + T * step) / T;
                 if (t < best) {
                     best = t;
                     *plan = TilePlan{T, H, TJ, cpw};
