@@ -261,6 +261,20 @@ int build_mask(const llb_desc* d, int ld, std::vector<uint8_t>& mask, std::vecto
     return LLB_OK;
 }
 
+// Whether open nodes stand above one another, on the left or right side.  In
+// FP16 tiles a lane closes its four rows there one after the other; the cluster
+// kernel, a node per thread, then steps longer runs of lattices of few nodes
+// faster, shorter ones not (its launch takes 8 us): us a step, cluster / tiles,
+// porous 90 x 95 runs of 3 4.1 / 3.0, of 8 2.8 / 2.8, of 200 2.0 / 2.7, 110 x 110
+// of 200 2.2 / 2.7, 120 x 130 of 200 2.7 / 2.7, 150 x 165 of 200 3.1 / 2.75; a
+// cavity of 90 x 92 of 200 2.15 / 1.9.
+bool open_on_sides(const llb_desc* d) {
+    auto any = [](const int32_t* side, int64_t n) {
+        return side && std::any_of(side, side + n, [](int32_t s) { return s == SIDE_LEFT || s == SIDE_RIGHT; });
+    };
+    return any(d->inlet_side, d->n_inlet) || any(d->outlet_side, d->n_outlet);
+}
+
 int ensure_partials(llb_handle h, int nblocks) {
     if (h->partial_blocks >= nblocks) return LLB_OK;
     if (h->d_partials) { dev_free(h, h->d_partials); h->d_partials = nullptr; }
@@ -351,9 +365,11 @@ int run_config(llb_handle h, int32_t plain) {
     return h->group_min > 0 && plain >= h->group_min ? FIRST_STREAM_CONFIG : h->tma_cfg;
 }
 
-// Whether llb_step of `nsteps` steps, the last of them an output step if
-// `macro`, runs in tiles.
-bool run_in_tiles(llb_handle h, int32_t, bool) { return h->tile.T > 0; }
+// Whether llb_step of `nsteps` steps runs in tiles (except for steps that
+// tile_steps leaves to the one-step kernel).
+bool run_in_tiles(llb_handle h, int32_t nsteps) {
+    return h->tile.T > 0 && (h->tile.longest == 0 || nsteps <= h->tile.longest);
+}
 
 // The lattice's default way of stepping, kept beside the configuration in use.
 void keep_default(llb_handle h) {
@@ -615,11 +631,16 @@ int launch_one(llb_handle h, int cfg, bool macro, long long graph_offset = -1) {
     return LLB_OK;
 }
 
-// Steps of the next launch of a lattice that steps in tiles, `left` to go:
-// evenly split.
-int32_t tile_steps(llb_handle h, int32_t left) {
-    const int32_t launches = (left + h->tile.T - 1) / h->tile.T;
-    return (left + launches - 1) / launches;
+// Steps of the next launch of a lattice that steps in tiles, `left` to go, the
+// last an output step if `macro`: evenly split, but a full launch where that
+// would leave launches too short to be worth it; 0 for a lone step of the
+// one-step kernel.
+int32_t tile_steps(llb_handle h, int32_t left, bool macro) {
+    const TilePlan& p = h->tile;
+    if (macro && p.lone_output) --left;
+    if (left < p.least) return 0;
+    const int32_t launches = (left + p.T - 1) / p.T;
+    return left / launches < p.least ? p.T : (left + launches - 1) / launches;
 }
 
 // nsteps steps of a lattice that steps in tiles; with macro the last one writes
@@ -628,9 +649,14 @@ int step_tiles(llb_handle h, int32_t nsteps, bool macro) {
     int rc = state_to_dense(h);
     if (rc) return rc;
     for (int32_t left = nsteps; left > 0;) {
-        const int32_t k = tile_steps(h, left);
-        const bool out = macro && k == left;
-        cudaError_t e = launch_step_tile(h->storage, make_ctx(h), h->tile, h->f[h->cur], h->f[h->cur ^ 1], k, out);
+        const int32_t k = tile_steps(h, left, macro);
+        if (k == 0) {
+            if ((rc = launch_one(h, PIPE_GRID, macro && left == 1))) return rc;
+            --left;
+            continue;
+        }
+        cudaError_t e = launch_step_tile(h->storage, make_ctx(h), h->tile, h->f[h->cur], h->f[h->cur ^ 1], k,
+                                         macro && k == left);
         if (e != cudaSuccess) return cuda_fail(h, e, "tile step kernel launch");
         h->cur ^= 1;
         h->step += k;
@@ -918,6 +944,8 @@ int llb_create(const llb_desc* d, llb_handle* out) {
     if (h->group_min == 0 && (h->tma_cfg == PIPE_GRID || h->tma_cfg == PIPE_CLUSTER))
         (void)tile_plan(h->storage, static_cast<int>(h->R), static_cast<int>(h->C), !ps.empty(),
                         h->tma_cfg == PIPE_CLUSTER, h->sm_count, &h->tile);
+    if (h->tma_cfg == PIPE_CLUSTER && h->storage == LLB_STORE_F16S && h->R * h->C < 16000 && open_on_sides(d))
+        h->tile.longest = 8;
     keep_default(h);
     staging_add_user();
     h->staging_user = true;
@@ -975,7 +1003,7 @@ int llb_step(llb_handle h, int32_t nsteps, uint32_t flags) {
     int rc = select_device(h);
     if (rc) return rc;
     const bool macro = (flags & LLB_STEP_MACRO) != 0;
-    if (run_in_tiles(h, nsteps, macro)) return step_tiles(h, nsteps, macro);
+    if (run_in_tiles(h, nsteps)) return step_tiles(h, nsteps, macro);
     int32_t plain = macro ? nsteps - 1 : nsteps;
     const int cfg = run_config(h, plain);
     const bool compact = cfg == PIPE_COMPACT;
@@ -1324,9 +1352,10 @@ int llb_reset_pipeline(llb_handle h) {
 int llb_run_kernel(llb_handle h, int32_t nsteps, uint32_t flags, int32_t* config, int32_t* per_launch) {
     if (!h || nsteps < 1 || !config || !per_launch) return fail(h, LLB_E_INVALID, "bad arguments");
     const bool macro = (flags & LLB_STEP_MACRO) != 0;
-    if (run_in_tiles(h, nsteps, macro)) {
-        *config = LLB_KERNEL_TILES;
-        *per_launch = tile_steps(h, nsteps);
+    if (run_in_tiles(h, nsteps)) {
+        const int32_t k = tile_steps(h, nsteps, macro);
+        *config = k > 0 ? LLB_KERNEL_TILES : PIPE_GRID;
+        *per_launch = std::max(k, 1);
         return LLB_OK;
     }
     const int32_t plain = macro ? nsteps - 1 : nsteps;

@@ -78,6 +78,9 @@ cudaError_t launch_step_stream(int storage, int cfg, const LaunchCtx& ctx, const
 // columns per warp.
 struct TilePlan {
     int T = 0, H = 0, TJ = 0, CPW = 1;
+    int least = 2;             // steps a launch has to take to be worth it
+    bool lone_output = false;  // output steps run on the one-step kernel
+    int longest = 0;           // runs of more steps do not take the tiles (0: any)
 };
 // False: one step a launch.  cluster: the lattice's one-step default is the
 // cluster kernel.

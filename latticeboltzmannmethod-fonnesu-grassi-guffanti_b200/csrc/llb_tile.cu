@@ -73,6 +73,16 @@ cudaError_t step_tile(const LaunchCtx& x, const TilePlan& p, const void* fin, vo
 // 3.60, TRT 3.44 / 3.82) and not against the cluster kernel, whose lattices need
 // them only when they are a few rows high, most of a tile outside (3 x 3900 FP64
 // 2.1 / 4.1, FP32 1.9 / 5.0; 8 x 3000 FP16 1.17 times the cluster's).
+//
+// A launch costs its load and its halo however few steps it takes.  us a step,
+// one-step kernels / tiles: launches of one step FP64 181 x 333 3.9 / 4.9, FP16
+// 256 x 1024 6.4 / 8.3, FP64 129^2 3.4 / 3.2; of two, one column a warp, 129^2 3.4 /
+// 2.1; two columns FP64 1492 x 43 3.4 / 3.6, TRT 3.4 / 3.8, FP16 256 x 1024 6.4 /
+// 6.1; of three 3.4 / 3.1, TRT 3.4 / 3.35, 6.4 / 5.5.  So two steps at least, three
+// with two columns.  In FP16 a lane writes the
+// output of its four rows one after the other, 32 bytes apart across the warp,
+// which with two columns costs more than the one-step kernel's output step: a
+// run of two steps with output 256 x 1024 6.6 / 8.1, of three 6.5 / 7.0.
 bool tile_plan(int storage, int R, int C, bool partial, bool cluster, int sm_count, TilePlan* plan) {
     *plan = TilePlan{};
     const int form = partial ? 3 : storage == LLB_STORE_F64 ? 0 : storage == LLB_STORE_F32S ? 1 : 2;
@@ -93,7 +103,7 @@ bool tile_plan(int storage, int R, int C, bool partial, bool cluster, int sm_cou
                 const double t = (1.5 + T * step) / T;
                 if (t < best) {
                     best = t;
-                    *plan = TilePlan{T, H, TJ, cpw};
+                    *plan = TilePlan{T, H, TJ, cpw, cpw == 2 ? 3 : 2, form == 2 && cpw == 2};
                 }
             }
     return plan->T > 0;

@@ -1,5 +1,6 @@
 """Which lattices step in tiles: those with no more tiles than SMs, and not a few
 rows that the cluster kernel holds.  The numbers of tiles are for 148 SMs."""
+import numpy as np
 import pytest
 
 import harness as H
@@ -40,3 +41,45 @@ def test_lattices_that_step_in_tiles(rows, cols, form, tiles):
             assert 3 <= g.run_kernel(200)[1] <= 8
             g.set_pipeline(g.pipeline)
             assert kernel(g, 200) == g.pipeline
+
+
+# lattice, form, and the kernel of a run of so many steps (with output: o): T tiles,
+# G one thread per node, C the cluster
+RUNS = [("cavity 129 x 129", 0, dict(zip((1, 2, 3, 50, "1o", "2o", "3o"), "GTTTGTT"))),
+        ("cavity 181 x 333", 0, dict(zip((1, 2, 3, 50, "1o", "2o", "3o"), "GGTTGGT"))),
+        ("cavity 40 x 50", 1, dict(zip((1, 2, 3, 50, "1o", "2o", "3o"), "GTTTGTT"))),
+        ("cavity 256 x 1024", 2, dict(zip((1, 2, 3, 50, "1o", "2o", "3o", "4o"), "GGTTGGGT"))),
+        ("cavity 181 x 333", 2, dict(zip((1, 2, 3, 50, "1o", "2o", "3o"), "GTTTGTT"))),
+        ("cavity 90 x 92", 2, dict(zip((1, 2, 8, 9, 200, "1o", "2o"), "GTTTTGT"))),
+        ("channel 90 x 95", 2, dict(zip((1, 2, 8, 9, 200, "1o", "8o", "9o"), "GTTCCGTC"))),
+        ("channel 150 x 165", 2, dict(zip((1, 2, 8, 9, 200, "1o", "9o"), "GTTTTGT")))]
+
+
+@pytest.mark.parametrize("name,form,runs", RUNS, ids=[f"{r[0]} {r[1]}".replace(" ", "_") for r in RUNS])
+def test_short_runs(name, form, runs):
+    """Launches of one step, of two with two columns a warp, and long runs of small
+    FP16 channels stay on the one-step kernels; the bits are theirs."""
+    if sms() != 148:
+        pytest.skip("tiles per SM counted for 148 SMs")
+    kind, rows, _, cols = name.split()
+    rows, cols = int(rows), int(cols)
+    t = box(rows, cols) if kind == "cavity" else H.channel_types(rows, cols, discs=[(rows // 2, cols // 3, rows // 8)])
+    posts = []
+    for default in (True, False):
+        with lattice(t, storage=form) as g:
+            if not default:
+                g.set_pipeline(-1)
+            for run, k in runs.items():
+                n, out = (int(run[:-1]), True) if isinstance(run, str) else (run, False)
+                if default:
+                    assert kernel(g, n, out) == {"T": TILES, "G": -1, "C": -4}[k], run
+                g.step(n, macro=out)
+                if out:
+                    posts.append(g.macro()[1])
+            for n in (4, 5, 7, 10, 11):  # remainders
+                g.step(n, macro=n % 2 == 1)
+            assert g.t == 1 + 37 + sum(int(str(r).rstrip("o")) for r in runs)
+            posts += [g.post_collision(), g.macro()[0]]
+    half = len(posts) // 2
+    for a, b in zip(posts[:half], posts[half:]):
+        np.testing.assert_array_equal(a, b)
