@@ -4,6 +4,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -184,15 +186,44 @@ inline int default_pipeline(const llb_lattice& h) {
 //          FP16  1800^2 30.1 / 30.6, 2000^2 38.8 / 32.2, 4096^2 142 / 119
 // On the compacted pipeline only longer runs leave its planes: shorter ones
 // would pay for the copies between the layouts.
+//
+// The lines are for lattices of many rows.  A strip stores 28, 56 or 112 rows of
+// the 32, 64 or 128 it streams, a lattice of few rows streams a last strip that
+// is mostly outside, and the two edge strips, in chunks half as wide, cost 1.22
+// times an inner one.  The rows streamed, so weighed, over those of the one-step
+// kernels' 32-row blocks (on the compacted pipeline, which skips what is not
+// there, over the rows themselves) may be as many times more as streaming gains,
+// and a little more with every doubling of the lattice.  us a step, one-step
+// default / streaming (ratio of rows): FP64 64 x 25000 (1.72) 1.01 times, TRT 1.12
+// times as long; FP32 100 x 9000 (1.22) 0.97 times, 200 x 5000 (1.27) 1.02 times, 400 x 2100 (1.30) 11.1 / 11.6,
+// 128 x 8192 (1.72) 15.2 / 17.6, 64 x 14000 (2.4) 16.4 / 21.6; FP16 812^2 (1.30) 9.6 /
+// 9.0, 700 x 1000 (1.35) 1.02 times, 260 x 5000 (1.53) 1.02 times, 128 x 8192 (2.4)
+// 16.3 / 24.0; porous FP64 300 x 11000 (1.22) 0.96 times, 148 x 22317 (1.39) 62.0 /
+// 66.0, FP32 295 x 7464 (1.40) 26.4 / 24.1, 171 x 12877 (1.66) 27.1 / 27.7, FP16
+// 591 x 6520 (1.40) 39.4 / 36.1, 400 x 9800 (1.42) 1.01 times, 341 x 11300 (1.67)
+// 39.3 / 46.3.  Below 32 columns the four a task streams besides its own decide:
+// FP64 250000 x 3 13.7 / 18.6, 86016 x 8 12.3 / 13.8, FP32 68812 x 12 11.0 / 11.9,
+// FP16 131072 x 20 22.8 / 23.7.
 inline int default_group_min(const llb_lattice& h) {
-    if (h.d_ps || h.n_active == 0) return 0;
+    if (h.d_ps || h.n_active == 0 || h.C < 32) return 0;
     const int64_t n = h.R * h.C;
     const int form = h.storage == LLB_STORE_F64 ? 0 : h.storage == LLB_STORE_F32S ? 1 : 2;
     const bool trt64 = form == 0 && h.coll.model == 1;
     static constexpr int64_t kDense[3] = {5LL << 17, 6LL << 17, 5LL << 17};
     static constexpr int64_t kPorous[3] = {3LL << 20, 2LL << 20, 7LL << 19};
-    if (h.tma_cfg == PIPE_COMPACT) return n >= kPorous[form] && !trt64 ? 32 : 0;
-    return n >= (trt64 ? 6LL << 17 : kDense[form]) ? llb::STREAM_STEPS : 0;
+    const int64_t line = h.tma_cfg == PIPE_COMPACT ? kPorous[form] : trt64 ? 6LL << 17 : kDense[form];
+    if (n < line) return 0;
+    const int64_t strip = 32LL << form, strips = (h.R + strip - (4LL << form) - 1) / (strip - (4LL << form));
+    const double rows = (static_cast<double>(strips) + 0.22 * static_cast<double>(std::min<int64_t>(strips, 2))) *
+                        static_cast<double>(strip);
+    if (h.tma_cfg == PIPE_COMPACT) {
+        static constexpr double kMost[3] = {1.25, 1.45, 1.4};
+        return !trt64 && rows <= kMost[form] * static_cast<double>(h.R) ? 32 : 0;
+    }
+    static constexpr double kMost[3] = {1.45, 1.22, 1.33}, kMore[3] = {0.1, 0.12, 0.1};
+    const double most = (trt64 ? 1.3 : kMost[form]) +
+                        kMore[form] * std::log2(static_cast<double>(n) / static_cast<double>(line));
+    return rows <= std::min(most, 1.5) * static_cast<double>((h.R + 31) / 32 * 32) ? llb::STREAM_STEPS : 0;
 }
 
 namespace llb {
