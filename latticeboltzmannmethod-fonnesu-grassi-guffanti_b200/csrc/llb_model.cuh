@@ -242,9 +242,14 @@ struct Two {
         const float2 x = unpack(a);
         return pack(1.0f / x.x, 1.0f / x.y);
     }
+    // Both values in the range of inverse_mid.  The minimum and maximum that hand
+    // on a NaN: fminf and fmaxf return the other value.
     static __device__ __forceinline__ bool mid(V a) {
         const float2 x = unpack(a);
-        return fminf(x.x, x.y) > 0x1p-120f && fmaxf(x.x, x.y) < 0x1p120f;
+        float lo, hi;
+        asm("min.NaN.f32 %0, %1, %2;" : "=f"(lo) : "f"(x.x), "f"(x.y));
+        asm("max.NaN.f32 %0, %1, %2;" : "=f"(hi) : "f"(x.x), "f"(x.y));
+        return lo > 0x1p-120f && hi < 0x1p120f;
     }
 };
 
