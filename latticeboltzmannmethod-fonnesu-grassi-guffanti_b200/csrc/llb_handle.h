@@ -193,17 +193,22 @@ inline int default_pipeline(const llb_lattice& h) {
 // times an inner one.  The rows streamed, so weighed, over those of the one-step
 // kernels' 32-row blocks (on the compacted pipeline, which skips what is not
 // there, over the rows themselves) may be as many times more as streaming gains,
-// and a little more with every doubling of the lattice.  us a step, one-step
-// default / streaming (ratio of rows): FP64 64 x 25000 (1.72) 1.01 times, TRT 1.12
-// times as long; FP32 100 x 9000 (1.22) 0.97 times, 200 x 5000 (1.27) 1.02 times, 400 x 2100 (1.30) 11.1 / 11.6,
-// 128 x 8192 (1.72) 15.2 / 17.6, 64 x 14000 (2.4) 16.4 / 21.6; FP16 812^2 (1.30) 9.6 /
-// 9.0, 700 x 1000 (1.35) 1.02 times, 260 x 5000 (1.53) 1.02 times, 128 x 8192 (2.4)
-// 16.3 / 24.0; porous FP64 300 x 11000 (1.22) 0.96 times, 148 x 22317 (1.39) 62.0 /
-// 66.0, FP32 295 x 7464 (1.40) 26.4 / 24.1, 171 x 12877 (1.66) 27.1 / 27.7, FP16
-// 591 x 6520 (1.40) 39.4 / 36.1, 400 x 9800 (1.42) 1.01 times, 341 x 11300 (1.67)
-// 39.3 / 46.3.  Below 32 columns the four a task streams besides its own decide:
-// FP64 250000 x 3 13.7 / 18.6, 86016 x 8 12.3 / 13.8, FP32 68812 x 12 11.0 / 11.9,
-// FP16 131072 x 20 22.8 / 23.7.
+// and more with every doubling of the lattice.  us a step, one-step default /
+// streaming (ratio of rows):
+//   FP64  64 x 25000 (1.72) 1.01 times as long, TRT 1.12 times; 95 x 18000 (1.48)
+//         0.97, TRT 1.00 to 1.05
+//   FP32  100 x 9000 (1.22) 0.97, 200 x 5000 (1.27) 1.02, 400 x 2100 (1.30) 11.1 /
+//         11.6, 128 x 8192 (1.72) 15.2 / 17.6, 128 x 24000 (1.72) 0.96, 64 x 14000
+//         (2.4) 16.4 / 21.6
+//   FP16  812^2 (1.30) 9.6 / 9.0, 700 x 1000 (1.35) 1.02, 260 x 5000 (1.53) 1.02,
+//         260 x 16000 73.7 / 51.7, 85 x 30840 (1.63) 43.1 / 26.5, 128 x 8192 (2.4)
+//         16.3 / 24.0
+//   porous FP64 300 x 11000 (1.22) 0.96, 148 x 22317 (1.39) 62.0 / 66.0; FP32 295 x
+//         7464 (1.40) 26.4 / 24.1, 171 x 12877 (1.66) 27.1 / 27.7; FP16 591 x 6520
+//         (1.40) 39.4 / 36.1, 400 x 9800 (1.42) 1.01, 341 x 11300 (1.67) 39.3 / 46.3
+// Below 32 columns the four a task streams besides its own decide: FP64 250000 x 3
+// 13.7 / 18.6, 86016 x 8 12.3 / 13.8, FP32 68812 x 12 11.0 / 11.9, FP16 131072 x 20
+// 22.8 / 23.7.
 inline int default_group_min(const llb_lattice& h) {
     if (h.d_ps || h.n_active == 0 || h.C < 32) return 0;
     const int64_t n = h.R * h.C;
@@ -221,9 +226,9 @@ inline int default_group_min(const llb_lattice& h) {
         return !trt64 && rows <= kMost[form] * static_cast<double>(h.R) ? 32 : 0;
     }
     static constexpr double kMost[3] = {1.45, 1.22, 1.33}, kMore[3] = {0.1, 0.12, 0.1};
-    const double most = (trt64 ? 1.3 : kMost[form]) +
-                        kMore[form] * std::log2(static_cast<double>(n) / static_cast<double>(line));
-    return rows <= std::min(most, 1.5) * static_cast<double>((h.R + 31) / 32 * 32) ? llb::STREAM_STEPS : 0;
+    const double doublings = std::log2(static_cast<double>(n) / static_cast<double>(line));
+    const double most = trt64 ? 1.25 + 0.08 * doublings : kMost[form] + (kMore[form] + 0.08 * doublings) * doublings;
+    return rows <= std::min(most, 2.2) * static_cast<double>((h.R + 31) / 32 * 32) ? llb::STREAM_STEPS : 0;
 }
 
 namespace llb {

@@ -19,7 +19,8 @@ OPEN_FLOW = [(800, 819, F64, BGK, False), (800, 820, F64, BGK, True), (885, 888,
              (830, 789, F16, TRT, False), (830, 790, F16, BGK, True), (800, 820, F16, BGK, False),
              (100, 9000, F32, BGK, True), (400, 2100, F32, BGK, False), (128, 8192, F32, BGK, False), (64, 14000, F32, TRT, False),
              (128, 8192, F16, BGK, False), (440, 2100, F16, BGK, True), (128, 8192, F64, BGK, True),
-             (64, 14000, F64, TRT, False), (470, 6000, F16, BGK, True),
+             (64, 14000, F64, TRT, False), (470, 6000, F16, BGK, True), (260, 5000, F16, TRT, False), (260, 16000, F16, BGK, True),
+             (128, 16000, F32, BGK, False),
              (25000, 31, F64, BGK, False), (90000, 10, F32, BGK, False), (3, 60000, F16, BGK, False)]
 
 
