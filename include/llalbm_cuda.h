@@ -410,17 +410,20 @@ int llb_event_elapsed_ms(llb_handle h, int32_t slot_begin, int32_t slot_end, flo
    the form's default shape with the tile's bounce bytes loaded too), the
    two-steps-per-pass kernel (3..5: the intermediate step stays in registers,
    so a pair of steps reads and writes the populations once; a lone step runs
-   on the one-thread kernel), the one-thread-per-node kernel for
+   on the one-thread kernel; by default the longer runs of large lattices), the
+   one-thread-per-node kernel for
    config -1, for config -2 one thread per node of every 32-byte population
    sector that holds an active node (a list built on first use), for config -3
    one thread per slot of compacted planes that store only the fluid and open
    nodes (built on first use; the default for obstacle-rich lattices of 2^18
-   nodes or more), and for config -4 the lattice resident in the shared memory
+   nodes or more, which runs of 32 steps or more leave from 2 to 4 million
+   nodes), and for config -4 the lattice resident in the shared memory
    of one thread-block cluster of 16 blocks, up to 4096 steps per launch with
    a cluster barrier between steps (lattices whose column slabs fit: about
-   129 x 129 in FP64, 181 x 181 in FP32, 256 x 256 in FP16; the default up to
-   12 000 nodes, 26 000 in FP16).  Lattices with partially saturated
-   obstacles run on config -1 only; lattices beyond the 32-bit limits of the
+   129 x 129 in FP64, 181 x 181 in FP32, 256 x 256 in FP16; reported by default up
+   to 12 000 nodes, 26 000 in FP16, although most of these step in tiles).
+   Lattices with partially saturated obstacles take config -1 only; lattices
+   beyond the 32-bit limits of the
    sector list or the compacted tables (2^31 slots; neighbouring columns more
    than 65 535 slots apart) have no config -2 or -3, and lattices that do not
    fit a cluster have no config -4 (LLB_E_UNSUPPORTED).  A lattice in a batch
@@ -455,7 +458,8 @@ int llb_run_kernel(llb_handle h, int32_t nsteps, uint32_t flags, int32_t* config
    best and ms_per_step (either may be NULL) receive the choice and its time. */
 int llb_tune_pipeline(llb_handle h, int32_t trial_steps, int32_t* best, float* ms_per_step);
 /* Columns of lattice nodes per thread block of the one-thread-per-node kernel
-   (1..8; each block is 32 rows x block_y columns). */
+   (1..8; each block is 32 rows x block_y columns).  Runs on other kernels (llb_run_kernel)
+   do not change. */
 int llb_set_launch_shape(llb_handle h, int32_t block_y);
 /* Polls of the pipelined kernels' (configurations 0..6) waits for their
    shared-memory stages before they give up, flag LLB_E_TIMEOUT (read by

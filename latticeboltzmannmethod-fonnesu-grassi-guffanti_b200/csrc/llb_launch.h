@@ -65,7 +65,6 @@ cudaError_t launch_step_cluster_lowp(int storage, const LaunchCtx&, const Cluste
 // STREAM_STEPS plain steps per launch, streamed through registers
 // (llb_stream.cuh; configurations FIRST_STREAM_CONFIG .. +2).  pmap: the
 // population planes in boxes of stream_box_rows rows x 1 column x 9 planes.
-// False / an error for lattices beyond its 32-bit column offsets.
 constexpr int STREAM_STEPS = 2;
 constexpr int FIRST_STREAM_CONFIG = 3;
 constexpr bool is_stream(int cfg) { return cfg >= FIRST_STREAM_CONFIG && cfg < FIRST_STREAM_CONFIG + 3; }

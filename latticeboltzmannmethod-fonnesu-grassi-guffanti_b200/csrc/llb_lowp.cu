@@ -72,7 +72,7 @@ bool tma_plan_lowp(int storage, int cfg, TmaPlan* p) {
         case 0: fill_plan<ModelF32S, F32Cfg0>(0, p); return true;
         case 1: fill_plan<ModelF32S, F32Cfg1>(1, p); return true;
         case 2: fill_plan<ModelF32S, F32Cfg2>(2, p); return true;
-                    case 6: fill_plan<ModelF32S, F32Cfg6>(6, p); return true;
+        case 6: fill_plan<ModelF32S, F32Cfg6>(6, p); return true;
         default: return false;
         }
     }
@@ -93,7 +93,7 @@ cudaError_t launch_step_tma_lowp(int storage, const TmaPlan& p, const LaunchCtx&
         case 0: return do_step_tma<ModelF32S, F32Cfg0>(x, pm, mm, bm, fin, fout, grid);
         case 1: return do_step_tma<ModelF32S, F32Cfg1>(x, pm, mm, bm, fin, fout, grid);
         case 2: return do_step_tma<ModelF32S, F32Cfg2>(x, pm, mm, bm, fin, fout, grid);
-                    case 6: return do_step_tma<ModelF32S, F32Cfg6>(x, pm, mm, bm, fin, fout, grid);
+        case 6: return do_step_tma<ModelF32S, F32Cfg6>(x, pm, mm, bm, fin, fout, grid);
         default: return cudaErrorInvalidValue;
         }
     }

@@ -19,13 +19,13 @@ namespace {
 // Up to w = 40: the narrowest tasks that are one wave, none left over for a
 // second one.  Against tasks of 12 columns in several waves (us a step): channel
 // 1001 x 3005 FP32, w = 25, 26.4 -> 23.6; cavity 2048^2 FP16, w = 24, 32.1 -> 29.5;
-// porous 1300^2 FP64, w = 27, 31.8 -> 28.8; channel 1500 x 3000 FP32, w = 37, 37.1
-// -> 34.6.  Above, the slowest task of one wave takes too long (cavity 2400^2
-// FP32, w = 46, 48.3 in one wave): several waves, which the block scheduler
-// balances, of sqrt(9 w) columns up to 24 (porous 3600^2 FP32, w = 102, 98.7
-// against 101.9 in tasks of 17 columns; cavity 2900^2 FP32, w = 66, 58.5 against
-// 59.8 in tasks of 14), and of sqrt(3 w) when that is more (cavity 4096^2 FP64, w
-// = 258, 28 columns: 212 against 217 in tasks of 48 and 227 in tasks of 24).
+// porous 1300^2 FP64 on configuration 3, w = 27, 31.8 -> 28.8; channel 1500 x 3000
+// FP32, w = 37, 37.1 -> 34.6.  Above, the slowest task of one wave takes too long
+// (cavity 2400^2 FP32, w = 46, 48.3 in one wave): several waves, which the block
+// scheduler balances, of sqrt(9 w) columns up to 24 (porous 3600^2 FP32, w = 102,
+// 98.7 against 101.9 in tasks of 17 columns; cavity 2900^2 FP32, w = 66, 58.5
+// against 59.8 in tasks of 14), and of sqrt(3 w) when that is more (cavity 4096^2
+// FP64, w = 258, 28 columns: 212 against 217 in tasks of 48 and 227 in tasks of 24).
 // Edge strips (long path in every column) run chunks half as wide.
 template <class CFG>
 StreamTasks stream_tasks(int rows, int cols, long long ld, int sm_count) {

@@ -29,7 +29,9 @@
 // What bounds it (B200): FP64 HBM -- cavity 4096^2 212 us a step (two passes of
 // nine planes every two steps are 187 us at the copy bandwidth) against 335 us
 // for the tile-in-shared-memory kernel this one replaced; FP32 117 us against
-// 193 us, FP16 99 us against 141 us, there instruction issue.  The packed FP32
+// 193 us, FP16 99 us against 141 us, there fixed-latency waits at three and two
+// warps per scheduler (2048^2: issue slots 64 and 55 % busy, 1.4 cycles of wait
+// an instruction, DRAM 50 and 26 %; porous FP64 65 %, 1.7 and 55 %).  The packed FP32
 // arithmetic (Two, llb_model.cuh) halves the instructions of the shifted forms'
 // collision; without it FP32 ran 136 us.  Measured and dropped: four levels (the
 // state of four levels leaves 8 warps per SM, and FP64 needs 4 halo rows: 320 us,
