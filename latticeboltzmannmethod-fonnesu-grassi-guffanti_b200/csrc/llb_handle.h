@@ -186,7 +186,7 @@ inline int default_pipeline(const llb_lattice& h) {
 //          FP16  1800^2 30.1 / 30.6, 2000^2 38.8 / 32.2, 4096^2 142 / 119
 // On the compacted pipeline only longer runs leave its planes: shorter ones
 // would pay for the copies between the layouts, and stretches that alternate
-// still do (FP64 1775^2, runs of 32 and 8 in turn 57.3 / 58.3), so that line lies
+// still do (FP64 1775^2, runs of 32 and 8 in turn 57.4 / 58.3 to 60.2), so that line lies
 // above the size where a long run breaks even.  The other operator at the lines:
 // TRT FP32 890^2 9.6 / 8.9, FP16 900^2 11.3 / 10.6, porous FP32 1450^2 26.0 / 20.6,
 // FP16 1917^2 39.8 / 32.0.
